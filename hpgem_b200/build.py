@@ -22,11 +22,12 @@ SOURCES = sorted(glob.glob(os.path.join(CSRC, "*.cu"))) + [
     os.path.join(CSRC, "host", "setup.cpp"),
     os.path.join(CSRC, "host", "operators.cpp"),
     os.path.join(CSRC, "host", "linear.cpp"),
+    os.path.join(CSRC, "host", "lane.cpp"),
     os.path.join(CSRC, "host", "sources.cpp")]
 HEADERS = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(glob.glob(os.path.join(CSRC, "host", "*.h"))) + [
     os.path.join(CSRC, "host", "simplex_rules.inc"),
     os.path.join(os.path.dirname(HERE), "include", "hpgem_b200.h")]
-FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
+FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--split-compile=0", "-Xcompiler", "-fPIC"]
 
 
 def nvcc():

@@ -45,6 +45,13 @@ struct alignas(16) TensorItem {
     int slot;
 };
 template <typename KT>
+struct alignas(16) TensorLaneItem {
+    StageIOT<KT> io[2];
+    TensorLaneGeom g;
+    int64_t block0;  // first virtual block of kLaneWarps tiles
+    int slot;
+};
+template <typename KT>
 struct alignas(16) SliceItem {
     StageIOT<KT> io[2];
     const double *geo;
@@ -150,6 +157,26 @@ __global__ void __launch_bounds__(EPB *TensorConsts<P, DIM>::NB)
     }
 }
 
+// one element per thread, a warp per tile, kLaneWarps tiles per virtual block
+constexpr int kLaneWarps = 4;
+template <typename KT, int P, int DIM, int NIN, bool FIN>
+__global__ void __launch_bounds__(32 * kLaneWarps)
+    grouped_tensor_lane(const TensorLaneItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
+                        const int *remaining) {
+    const int n = *n_items;
+    const int64_t nb = *total;
+    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+        const int i = find_item(total, n, vb);
+        const int slot = items[i].slot;
+        __syncthreads();
+        if (remaining[slot] <= 0) continue;
+        __shared__ TensorLaneItem<KT> s_it;
+        const TensorLaneItem<KT> &it = item_to_shared(items, i, s_it);
+        const int64_t tile = (vb - it.block0) * kLaneWarps + (threadIdx.x >> 5);
+        if (tile < it.g.n_tiles) tensor_lane_body<KT, P, DIM, NIN, FIN>(it.io[parity[slot]], it.g, tile);
+    }
+}
+
 template <typename KT, int NIN, int NFIN>
 __global__ void __launch_bounds__(SliceShape::THREADS, sizeof(KT) == 4 ? 5 : (NFIN == 0 ? 5 : 4))
     grouped_slice(const SliceItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
@@ -247,7 +274,8 @@ __global__ void batch_set_slot(int *parity, int *remaining, int slot, int nsteps
 
 namespace {
 
-enum BatchKind { KIND_DENSE = 0, KIND_TENSOR = 1, KIND_SLICE = 2, KIND_LINEAR = 3, KIND_UMMA = 4, KIND_WAVE_TILES = 5 };
+enum BatchKind { KIND_DENSE = 0, KIND_TENSOR = 1, KIND_SLICE = 2, KIND_LINEAR = 3, KIND_UMMA = 4, KIND_WAVE_TILES = 5,
+                 KIND_TENSOR_LANE = 6 };
 
 struct BatchClass {
     // key
@@ -349,7 +377,7 @@ int batch_kind(const hgg_handle *h) {
     if (h->umma_tiles > 0) return KIND_UMMA;
     if (h->linear) return KIND_LINEAR;
     if (h->slice_ok) return KIND_SLICE;
-    if (h->op.tensor) return KIND_TENSOR;
+    if (h->op.tensor) return h->lane ? KIND_TENSOR_LANE : KIND_TENSOR;
     // the same choice as the handle's own dense launch: tiles where the contraction is FP64
     if (group_wave_wanted(h)) return KIND_WAVE_TILES;
     // Above 24 basis functions a batch takes the 16-element tiles on any member that
@@ -382,6 +410,7 @@ int64_t item_blocks(const BatchClass &c, const hgg_handle *h) {
     if (c.kind == KIND_UMMA) return h->umma_tiles;
     if (c.kind == KIND_WAVE_TILES) return h->group_tiles;
     if (c.kind == KIND_SLICE) return (nE + SliceShape::TE - 1) / SliceShape::TE;
+    if (c.kind == KIND_TENSOR_LANE) return (h->tlane.n_tiles + kLaneWarps - 1) / kLaneWarps;
     if (c.kind == KIND_TENSOR) {
         const int epb = tensor_epb(c.order, c.dim);
         return (nE + epb - 1) / epb;
@@ -393,6 +422,7 @@ size_t class_item_bytes(const BatchClass &c) {
     if (c.kind == KIND_DENSE || c.kind == KIND_WAVE_TILES)
         return c.mixed ? sizeof(DenseItem<float>) : sizeof(DenseItem<double>);
     if (c.kind == KIND_TENSOR) return c.mixed ? sizeof(TensorItem<float>) : sizeof(TensorItem<double>);
+    if (c.kind == KIND_TENSOR_LANE) return c.mixed ? sizeof(TensorLaneItem<float>) : sizeof(TensorLaneItem<double>);
     if (c.kind == KIND_LINEAR) return c.mixed ? sizeof(LinearItem<float>) : sizeof(LinearItem<double>);
     if (c.kind == KIND_UMMA) return sizeof(UmmaItem);
     return c.mixed ? sizeof(SliceItem<float>) : sizeof(SliceItem<double>);
@@ -437,6 +467,14 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
         it.block0 = block0;
         it.slot = slot;
         std::memcpy(dst, &it, sizeof(it));
+    } else if (c.kind == KIND_TENSOR_LANE) {
+        TensorLaneItem<KT> it{};
+        for (int par = 0; par < 2; ++par)
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+        it.g = h->tlane;
+        it.block0 = block0;
+        it.slot = slot;
+        std::memcpy(dst, &it, sizeof(it));
     } else if (c.kind == KIND_TENSOR) {
         TensorItem<KT> it{};
         for (int par = 0; par < 2; ++par)
@@ -466,6 +504,7 @@ void set_block0(const BatchClass &c, unsigned char *dst, int64_t block0) {
     if (c.kind == KIND_DENSE || c.kind == KIND_WAVE_TILES) put((DenseItem<KT> *)nullptr);
     else if (c.kind == KIND_UMMA) put((UmmaItem *)nullptr);
     else if (c.kind == KIND_LINEAR) put((LinearItem<KT> *)nullptr);
+    else if (c.kind == KIND_TENSOR_LANE) put((TensorLaneItem<KT> *)nullptr);
     else if (c.kind == KIND_TENSOR) put((TensorItem<KT> *)nullptr);
     else put((SliceItem<KT> *)nullptr);
 }
@@ -612,6 +651,26 @@ void launch_grouped_tensor(const hgg_batch *b, const BatchClass &c, int st, unsi
                      b->d_remaining, tc);
 }
 
+// stage-input vectors of a class's stage (the tableau's nonzero a_ij)
+int class_nin(const BatchClass &c, int st) {
+    int n = 0;
+    for (int j = 0; j < st; ++j) n += c.rk_a[st * c.S + j] != 0.0;
+    return n;
+}
+
+template <typename KT>
+void launch_grouped_tensor_lane(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
+    tensor_lane_dispatch(c.dim, c.order, [&](auto p, auto d) {
+        lane_stage_shape(class_nin(c, st), st == c.S - 1, [&](auto nin, auto fin) {
+            class_kernel(b,
+                         grouped_tensor_lane<KT, decltype(p)::value, decltype(d)::value, decltype(nin)::value,
+                                             decltype(fin)::value>,
+                         grid, 32 * kLaneWarps, 0, s, static_cast<const TensorLaneItem<KT> *>(c.d_items[st]), c.d_n,
+                         c.d_total, b->d_parity, b->d_remaining);
+        });
+    });
+}
+
 template <typename KT>
 void launch_grouped_slice(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
     SliceOps sops;
@@ -727,6 +786,9 @@ void launch_class_stage(hgg_batch *b, const BatchClass &c, int st, cudaStream_t 
                 c.mixed ? launch_grouped_wave<float, 3, 6>(b, c, st, grid, s) : launch_grouped_wave<double, 3, 6>(b, c, st, grid, s);
                 break;
         }
+    } else if (c.kind == KIND_TENSOR_LANE) {
+        if (c.mixed) launch_grouped_tensor_lane<float>(b, c, st, grid, s);
+        else launch_grouped_tensor_lane<double>(b, c, st, grid, s);
     } else if (c.kind == KIND_TENSOR) {
 #define HGG_GT(P)                                                  \
     case P:                                                        \

@@ -110,6 +110,42 @@ __global__ void convert_vector(const float *src, double *dst, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         dst[i] = (double)src[i];
 }
+// a vector from one layout to the other (to tiled or from tiled), element by element
+template <typename T>
+__global__ void relayout(const T *src, T *dst, int nb, int64_t n, bool tiled) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = i / nb;
+        const int k = (int)(i - e * nb);
+        dst[device_index(e, k, nb, tiled)] = src[device_index(e, k, nb, !tiled)];
+    }
+}
+
+int upload_tensor_geometry(hgg_handle *h);
+
+// moves every vector of a handle with a lane kernel between that kernel's layout and the
+// general kernels' (a change of the kernel variant; the padding elements stay zero)
+int set_lane_layout(hgg_handle *h, bool lane) {
+    int rc;
+    if (!lane && (rc = upload_tensor_geometry(h))) return rc;
+    auto move = [&](auto *v) {
+        using T = std::remove_pointer_t<decltype(v)>;
+        T *tmp = reinterpret_cast<T *>(h->d_scratch);
+        cudaMemsetAsync(tmp, 0, sizeof(T) * h->N_alloc, h->stream);
+        relayout<T><<<4 * h->num_sms, 256, 0, h->stream>>>(v, tmp, coefficients(h), h->N, lane);
+        cudaMemcpyAsync(v, tmp, sizeof(T) * h->N_alloc, cudaMemcpyDeviceToDevice, h->stream);
+        h->launches++;
+    };
+    for (int i = 0; i < 2; ++i) move(h->sol[i]);
+    for (void *k : h->k) {
+        if (h->mixed) move(static_cast<float *>(k));
+        else move(static_cast<double *>(k));
+    }
+    HGG_CUDA(h, cudaGetLastError());
+    HGG_CUDA(h, cudaStreamSynchronize(h->stream));
+    h->lane = h->tiled = lane;
+    return 0;
+}
+
 int launch_stage(hgg_handle *h, const StageIO &io) {
     int rc;
     if (h->linear) rc = launch_stage_linear(h, io);
@@ -289,6 +325,34 @@ int init_device_vectors(hgg_handle *h) {
 // tcgen05 tiles
 int attach_linear(hgg_handle *h, const LinearSystem &sys, int tiles_only = 0);
 
+// geometry of the general sum-factorised kernels (one-shot and pipelined): uploaded when
+// the handle is made, or for a handle with a lane kernel when another variant is asked for
+int upload_tensor_geometry(hgg_handle *h) {
+    const HostOperators &op = h->op;
+    if (h->d_pgeo) return 0;
+    int rc;
+    const int64_t n_pad = h->N_alloc / coefficients(h);
+    if ((rc = upload(h, op.elem_geo, &h->d_ahat)) || (rc = upload(h, op.t_nbr, &h->d_tnbr)) ||
+        (rc = upload(h, op.t_mode, &h->d_tmode)) || (rc = upload(h, op.t_sigma, &h->d_tsigma)))
+        return rc;
+    // packed geometry records of the pipelined kernel, padded to whole tiles:
+    // ahat[dim], sigma[2 dim] (double), nbr[2 dim] (int32), mode[2 dim] (int8)
+    const int d = op.dim, ns = 2 * d, gb = pipe_geo_bytes(d);
+    std::vector<unsigned char> pg((size_t)n_pad * gb, 0);
+    for (int64_t e = 0; e < op.nE; ++e) {
+        unsigned char *r = &pg[(size_t)e * gb];
+        double *dd = reinterpret_cast<double *>(r);
+        for (int c = 0; c < d; ++c) dd[c] = op.elem_geo[e * d + c];
+        for (int s2 = 0; s2 < ns; ++s2) dd[d + s2] = op.t_sigma[e * ns + s2];
+        int32_t *ni = reinterpret_cast<int32_t *>(r + 8 * (d + ns));
+        for (int s2 = 0; s2 < ns; ++s2) ni[s2] = op.t_nbr[e * ns + s2];
+        int8_t *mi = reinterpret_cast<int8_t *>(r + 8 * (d + ns) + 4 * ns);
+        for (int s2 = 0; s2 < ns; ++s2) mi[s2] = op.t_mode[e * ns + s2];
+    }
+    if ((rc = upload(h, pg, &h->d_pgeo))) return rc;
+    return 0;
+}
+
 // linear: the handle will run the stored-matrix kernel (attach_linear), so the
 // vectors stay in hpGEM order and the matrix-free operators are not uploaded
 int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = false) {
@@ -306,32 +370,24 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
     h->tile_elems = op.tensor ? pipe_tile_elems(op.order, op.dim) : 1;
     h->tensor_layout = op.tensor;
     h->slice_ok = op.tensor && op.dim == 3 && op.order == 3 && op.trace_pos[0] == 0 && op.trace_pos[1] == 1;
-    h->tiled = h->slice_ok;
+    std::vector<int32_t> lane_nbr;
+    h->lane_ok = h->lane = !h->slice_ok && tensor_lane_setup(op, h->tlane, lane_nbr);
+    h->tiled = h->slice_ok || h->lane;
     if (h->slice_ok) h->tile_elems = SliceShape::TE;
     if (h->mixed && !mixed_supported(h))
         return fail(h, HGG_ERR_UNSUPPORTED, "the FP32-mixed form has no kernel for this shape and order");
-    const int64_t n_pad = (op.nE + h->tile_elems - 1) / h->tile_elems * h->tile_elems;
+    int64_t n_pad = (op.nE + h->tile_elems - 1) / h->tile_elems * h->tile_elems;
+    if (h->lane_ok) n_pad = (n_pad + 31) / 32 * 32;  // whole tiles in either layout
     h->N_alloc = n_pad * op.V * op.nB;
     if ((rc = init_device_vectors(h))) return rc;
     if (op.tensor) {
-        if ((rc = upload(h, op.elem_geo, &h->d_ahat)) || (rc = upload(h, op.t_nbr, &h->d_tnbr)) ||
-            (rc = upload(h, op.t_mode, &h->d_tmode)) || (rc = upload(h, op.t_sigma, &h->d_tsigma)))
+        if (h->lane_ok) {
+            int32_t *d_nbr = nullptr;
+            if ((rc = upload(h, lane_nbr, &d_nbr))) return rc;
+            h->tlane.nbr = d_nbr;
+        } else if ((rc = upload_tensor_geometry(h))) {
             return rc;
-        // packed geometry records of the pipelined kernel, padded to whole tiles:
-        // ahat[dim], sigma[2 dim] (double), nbr[2 dim] (int32), mode[2 dim] (int8)
-        const int d = op.dim, ns = 2 * d, gb = pipe_geo_bytes(d);
-        std::vector<unsigned char> pg((size_t)n_pad * gb, 0);
-        for (int64_t e = 0; e < op.nE; ++e) {
-            unsigned char *r = &pg[(size_t)e * gb];
-            double *dd = reinterpret_cast<double *>(r);
-            for (int c = 0; c < d; ++c) dd[c] = op.elem_geo[e * d + c];
-            for (int s2 = 0; s2 < ns; ++s2) dd[d + s2] = op.t_sigma[e * ns + s2];
-            int32_t *ni = reinterpret_cast<int32_t *>(r + 8 * (d + ns));
-            for (int s2 = 0; s2 < ns; ++s2) ni[s2] = op.t_nbr[e * ns + s2];
-            int8_t *mi = reinterpret_cast<int8_t *>(r + 8 * (d + ns) + 4 * ns);
-            for (int s2 = 0; s2 < ns; ++s2) mi[s2] = op.t_mode[e * ns + s2];
         }
-        if ((rc = upload(h, pg, &h->d_pgeo))) return rc;
         if (h->slice_ok) {
             // slice kernel records, padded to whole tiles: ahat[3], sigma[6] (double),
             // nbr[6] (int32), mode[6] (int8), 2 bytes of padding
@@ -815,6 +871,9 @@ int hgg_set_kernel_variant(hgg_handle *h, int32_t variant) {
         return fail(h, HGG_ERR_UNSUPPORTED, "hexahedra of order 3 have one kernel organisation (the slice kernel)");
     if (variant != h->variant) {
         release_graphs(h);
+        int rc;
+        const bool lane = h->lane_ok && variant == 0;
+        if (lane != h->lane && (rc = set_lane_layout(h, lane))) return rc;
         h->variant = variant;
     }
     return 0;
@@ -839,7 +898,8 @@ int hgg_test_arm_without_copy(hgg_handle *h, int32_t polls) {
 namespace {
 constexpr int64_t kStaticScratchDoubles = int64_t(1) << 22;  // 32 MiB
 constexpr int kMaxStaticDevices = 64;
-static __device__ __align__(256) double g_static_scratch[kStaticScratchDoubles];
+// (a lane layout's last tile may reach a little further than the padding the limit counts)
+static __device__ __align__(256) double g_static_scratch[kStaticScratchDoubles + 4096];
 std::mutex g_static_mutex;
 double *g_static_ptr[kMaxStaticDevices] = {};
 }  // namespace
@@ -862,9 +922,10 @@ int hgg_time_derivative_static(hgg_handle *h, const double *u, double *k) {
         if (rc) return rc;
         return check_status(h);
     }
-    if (2 * h->N_alloc > kStaticScratchDoubles)
+    const int64_t counted = (h->op.nE + h->tile_elems - 1) / h->tile_elems * h->tile_elems * coefficients(h);
+    if (2 * counted > kStaticScratchDoubles)
         return fail(h, HGG_ERR_UNSUPPORTED,
-                    "problem needs " + std::to_string(2 * h->N_alloc) + " doubles of scratch; the static scratch holds " +
+                    "problem needs " + std::to_string(2 * counted) + " doubles of scratch; the static scratch holds " +
                         std::to_string(kStaticScratchDoubles) + " (" + std::to_string(kStaticScratchDoubles / 2) +
                         " per vector, padded to whole tiles)");
     double *base = nullptr;

@@ -14,6 +14,7 @@
 #include "dg_kernels.cuh"
 #include "linear_stage.cuh"
 #include "linear_umma.cuh"
+#include "tensor_lane.cuh"
 #include "tensor_pipe.cuh"
 #include "tensor_slice.cuh"
 #include "host/linear.h"
@@ -69,6 +70,10 @@ struct hgg_handle {
     // slice kernel (hexahedra, p = 3): per-element records of SliceShape::GR doubles
     bool slice_ok = false;
     double *d_slice_geo = nullptr;
+    // one-element-per-thread kernels (lane = element, tiled layout): the handle has one, and
+    // its vectors are in that kernel's layout (kernel variant 0)
+    bool lane_ok = false, lane = false;
+    hgg::TensorLaneGeom tlane{};
     // stored-matrix form (HpgemAPILinear): distinct folded matrices, transposed
     bool linear = false;
     int lin_R = 0, lin_slots = 0, lin_mats = 0;
@@ -143,6 +148,8 @@ int upload(hgg_handle *h, const std::vector<T> &v, T **dst) {
 }
 
 int alloc(hgg_handle *h, size_t bytes, void **dst);
+// coefficients per element (all variables)
+inline int coefficients(const hgg_handle *h) { return h->op.V * h->op.nB; }
 // the wave runs the grouped tile kernel (alone and in a batch): kernel variant 2, or
 // the automatic choice where it measured faster than the per-row kernel
 bool group_wave_wanted(const hgg_handle *h);

@@ -35,6 +35,23 @@ int launch_slice(hgg_handle *h, const StageIOT<KT> &io) {
     return 0;
 }
 
+// one element per thread: structured quadrilaterals, hexahedra of order 1 and 2
+template <typename KT>
+int launch_tensor_lane(hgg_handle *h, const StageIOT<KT> &io) {
+    const TensorLaneGeom &g = h->tlane;
+    // one warp per block until every SM has a block of four: a small mesh then spreads
+    // over all SMs
+    const int warps = g.n_tiles >= 8 * h->num_sms ? 4 : 1;
+    const unsigned blocks = (unsigned)((g.n_tiles + warps - 1) / warps);
+    const bool ok = tensor_lane_dispatch(h->op.dim, h->op.order, [&](auto p, auto d) {
+        lane_stage_shape(io.nin, io.unew != nullptr, [&](auto nin, auto fin) {
+            tensor_lane<KT, decltype(p)::value, decltype(d)::value, decltype(nin)::value, decltype(fin)::value>
+                <<<blocks, 32 * warps, 0, h->stream>>>(io, g);
+        });
+    });
+    return ok ? 0 : fail(h, HGG_ERR_UNSUPPORTED, "lane kernel: order out of range");
+}
+
 // shared memory of the pipelined kernel for a ring of `nbuf` slots of `nv` vectors
 template <int P, int DIM>
 size_t pipe_smem(int nbuf, int nv) {
@@ -145,6 +162,7 @@ int launch_tensor_oneshot_f(hgg_handle *h, const StageIOT<float> &io) {
 
 int launch_stage_tensor(hgg_handle *h, const StageIO &io) {
     if (h->slice_ok) return launch_slice<double>(h, io);
+    if (h->lane) return launch_tensor_lane(h, io);
     return h->op.dim == 2 ? launch_tensor_dim<2>(h, io)
                           : (h->op.dim == 3 ? launch_tensor_dim<3>(h, io)
                                             : fail(h, HGG_ERR_UNSUPPORTED, "tensor kernel needs dim 2 or 3"));
@@ -152,6 +170,7 @@ int launch_stage_tensor(hgg_handle *h, const StageIO &io) {
 
 int launch_stage_tensor(hgg_handle *h, const StageIOT<float> &io) {
     if (h->slice_ok) return launch_slice(h, io);
+    if (h->lane) return launch_tensor_lane(h, io);
     return h->op.dim == 2 ? launch_tensor_oneshot_f<2>(h, io)
                           : (h->op.dim == 3 ? launch_tensor_oneshot_f<3>(h, io)
                                             : fail(h, HGG_ERR_UNSUPPORTED, "tensor kernel needs dim 2 or 3"));

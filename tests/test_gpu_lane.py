@@ -1,0 +1,75 @@
+"""GPU: the one-element-per-thread kernels (tiled layout, the automatic choice on
+structured meshes) against the general kernels they replace there (kernel variant 1), at
+element counts around a tile of 32, along-axis and mixed-sign velocities, tableaux with
+zero, one and several vectors in a stage input, and after a change of the variant between
+steps.
+
+Both kernels evaluate the same operator from the same 64-bit geometry; the lane kernels
+fold it into fewer matrices first, so they differ by rounding only: 1e-12 of the largest
+coefficient as in the parity tests, in the FP32 form 2e-6 (a few FP32 roundings, 6e-8
+each, per step and stage over the steps taken here, damped by dt)."""
+import numpy as np
+import pytest
+
+import hpgem_b200
+from hpgem_b200 import _native
+
+pytestmark = pytest.mark.gpu
+
+RTOL = {_native.PRECISION_FP64: 1e-12, _native.PRECISION_FP32: 2e-6}
+
+
+def rel_err(a, b):
+    return float(np.abs(a - b).max() / np.abs(b).max())
+
+
+def solver(cells, order, a, tableau, precision):
+    s = hpgem_b200.Advection(len(cells), order, a, tableau=tableau, precision=precision)
+    d = len(cells)
+    return s.readMesh(hpgem_b200.structured_description(cells, [0.0] * d, [1.0] * d, False, True))
+
+
+# (cells, velocity): one tile not quite full, exactly full, one element more; several blocks; 3D
+QUADS = [([5, 6], [0.7, -0.4]), ([8, 4], [-0.3, 0.9]), ([11, 3], [1.0, 0.0]), ([67, 71], [0.0, -1.0])]
+HEXES = [([3, 3, 3], [0.5, -0.6, 0.7]), ([4, 4, 2], [-1.0, 0.0, 0.3]), ([11, 9, 13], [0.2, 0.3, 0.9])]
+
+
+@pytest.mark.parametrize("precision", [_native.PRECISION_FP64, _native.PRECISION_FP32])
+@pytest.mark.parametrize("tableau", ["ForwardEuler", "RK4_4", "DormandPrince"])
+@pytest.mark.parametrize("cells,a,order", [(c, a, p) for c, a in QUADS for p in (1, 2, 3, 4, 5)] +
+                         [(c, a, p) for c, a in HEXES for p in (1, 2)])
+def test_tensor_lane_matches_the_one_shot_kernel(cells, a, order, tableau, precision):
+    res = {}
+    for variant in (0, 1):
+        s = solver(cells, order, a, tableau, precision)
+        s.handle.set_kernel_variant(variant)
+        assert s.handle.kernel_kind == "tensor"
+        u0 = np.random.default_rng(order).standard_normal(s.handle.vector_length)
+        s.handle.set_state(0, u0)
+        assert np.array_equal(s.handle.get_state(0), u0)
+        h = 1.0 / max(cells)
+        s.handle.step(0.0, 0.02 * h / (2 * order + 1) ** 2, 3)
+        stages = 7 if tableau == "DormandPrince" else 4 if tableau == "RK4_4" else 1
+        res[variant] = [s.handle.get_state(v) for v in range(stages + 1)]
+    assert rel_err(res[0][0], res[1][0]) < RTOL[precision]
+    for k0, k1 in zip(res[0][1:], res[1][1:]):  # the stage vectors are k / dt larger: their own rounding
+        assert rel_err(k0, k1) < (1e-12 if precision == _native.PRECISION_FP64 else 5e-6)
+
+
+@pytest.mark.parametrize("precision", [_native.PRECISION_FP64, _native.PRECISION_FP32])
+def test_variant_change_keeps_every_vector(precision):
+    s = solver([13, 9], 3, [0.8, -0.5], "RK4_4", precision)
+    h = s.handle
+    h.set_state(0, np.random.default_rng(3).standard_normal(h.vector_length))
+    h.step(0.0, 1e-4, 2)
+    before = [h.get_state(v) for v in range(5)]
+    for variant in (1, 2, 0):
+        h.set_kernel_variant(variant)
+        for v in range(5):
+            assert np.array_equal(h.get_state(v), before[v])
+    h.step(0.0, 1e-4, 1)
+    mixed = h.get_state(0)
+    t = solver([13, 9], 3, [0.8, -0.5], "RK4_4", precision)
+    t.handle.set_state(0, before[0])
+    t.handle.step(0.0, 1e-4, 1)
+    assert np.array_equal(mixed, t.handle.get_state(0))
