@@ -70,7 +70,8 @@ class Batch:
         return int(self._lib.hgg_batch_num_classes(self._raw))
 
     KINDS = {0: "dense", 1: "sum-factorised", 2: "sum-factorised slices", 3: "stored-matrix tiles",
-             4: "tensor-core tiles", 5: "wave tiles", 6: "sum-factorised lanes"}
+             4: "tensor-core tiles", 5: "wave tiles", 6: "sum-factorised lanes",
+             7: "lane tables"}
 
     def class_info(self):
         """One dict per kernel class with members: kernel kind, shape, dim, order, physics,

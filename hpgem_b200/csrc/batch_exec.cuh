@@ -52,6 +52,13 @@ struct alignas(16) TensorLaneItem {
     int slot;
 };
 template <typename KT>
+struct alignas(16) LaneItem {
+    StageIOT<KT> io[2];
+    LaneGeom g;
+    int64_t block0;  // first virtual block (= chunk)
+    int slot;
+};
+template <typename KT>
 struct alignas(16) SliceItem {
     StageIOT<KT> io[2];
     const double *geo;
@@ -177,6 +184,41 @@ __global__ void __launch_bounds__(32 * kLaneWarps)
     }
 }
 
+// simplices and the wave, one element per thread: a chunk of a member per virtual block
+template <typename KT, typename CT, typename ST, int DIM, int NFL, int NB>
+__global__ void __launch_bounds__(LaneShape<KT, CT, DIM, NFL, NB, true>::THREADS)
+    grouped_wave_lane(const LaneItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
+                      const int *remaining) {
+    const int n = *n_items;
+    const int64_t nb = *total;
+    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+        const int i = find_item(total, n, vb);
+        const int slot = items[i].slot;
+        __syncthreads();
+        if (remaining[slot] <= 0) continue;
+        __shared__ LaneItem<KT> s_it;
+        const LaneItem<KT> &it = item_to_shared(items, i, s_it);
+        wave_lane_body<KT, CT, ST, DIM, NFL, NB>(it.io[parity[slot]], it.g, vb - it.block0);
+    }
+}
+
+template <typename KT, typename CT, int DIM, int NFL, int NB, int NIN>
+__global__ void __launch_bounds__(LaneShape<KT, CT, DIM, NFL, NB, false>::THREADS)
+    grouped_advection_lane(const LaneItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
+                           const int *remaining) {
+    const int n = *n_items;
+    const int64_t nb = *total;
+    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+        const int i = find_item(total, n, vb);
+        const int slot = items[i].slot;
+        __syncthreads();
+        if (remaining[slot] <= 0) continue;
+        __shared__ LaneItem<KT> s_it;
+        const LaneItem<KT> &it = item_to_shared(items, i, s_it);
+        advection_lane_body<KT, CT, DIM, NFL, NB, NIN>(it.io[parity[slot]], it.g, vb - it.block0);
+    }
+}
+
 template <typename KT, int NIN, int NFIN>
 __global__ void __launch_bounds__(SliceShape::THREADS, sizeof(KT) == 4 ? 5 : (NFIN == 0 ? 5 : 4))
     grouped_slice(const SliceItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
@@ -275,7 +317,7 @@ __global__ void batch_set_slot(int *parity, int *remaining, int slot, int nsteps
 namespace {
 
 enum BatchKind { KIND_DENSE = 0, KIND_TENSOR = 1, KIND_SLICE = 2, KIND_LINEAR = 3, KIND_UMMA = 4, KIND_WAVE_TILES = 5,
-                 KIND_TENSOR_LANE = 6 };
+                 KIND_TENSOR_LANE = 6, KIND_LANE = 7 };
 
 struct BatchClass {
     // key
@@ -289,6 +331,7 @@ struct BatchClass {
     std::vector<double> rk_a, rk_b;
     // members and launch shape
     std::vector<int> slots;
+    int lane_bytes = 0;   // lane kernels of simplices and the wave: bytes of a group's table
     int epb = 1;          // dense: elements per block
     int ctas_per_sm = 2;  // persistent CTAs per SM
     bool tuned = false;
@@ -374,6 +417,7 @@ int bfail(hgg_batch *b, int code, const std::string &msg) {
     } while (0)
 
 int batch_kind(const hgg_handle *h) {
+    if (h->lane && !h->op.tensor) return KIND_LANE;
     if (h->umma_tiles > 0) return KIND_UMMA;
     if (h->linear) return KIND_LINEAR;
     if (h->slice_ok) return KIND_SLICE;
@@ -394,6 +438,7 @@ bool same_class(const BatchClass &c, const hgg_handle *h) {
     return c.kind == batch_kind(h) && c.shape == h->op.shape && c.order == h->op.order && c.dim == h->op.dim &&
            c.physics == h->op.physics && c.mixed == h->mixed && c.S == h->S && c.rk_a == h->rk_a &&
            c.rk_b == h->rk_b &&
+           (c.kind != KIND_LANE || c.rep.nB == h->op.nB) &&
            (c.kind != KIND_UMMA || (c.precision == h->precision && c.rows == h->lin_R && c.lslots == h->lin_slots));
 }
 
@@ -410,6 +455,7 @@ int64_t item_blocks(const BatchClass &c, const hgg_handle *h) {
     if (c.kind == KIND_UMMA) return h->umma_tiles;
     if (c.kind == KIND_WAVE_TILES) return h->group_tiles;
     if (c.kind == KIND_SLICE) return (nE + SliceShape::TE - 1) / SliceShape::TE;
+    if (c.kind == KIND_LANE) return h->lgeo.n_chunks;
     if (c.kind == KIND_TENSOR_LANE) return (h->tlane.n_tiles + kLaneWarps - 1) / kLaneWarps;
     if (c.kind == KIND_TENSOR) {
         const int epb = tensor_epb(c.order, c.dim);
@@ -422,6 +468,7 @@ size_t class_item_bytes(const BatchClass &c) {
     if (c.kind == KIND_DENSE || c.kind == KIND_WAVE_TILES)
         return c.mixed ? sizeof(DenseItem<float>) : sizeof(DenseItem<double>);
     if (c.kind == KIND_TENSOR) return c.mixed ? sizeof(TensorItem<float>) : sizeof(TensorItem<double>);
+    if (c.kind == KIND_LANE) return c.mixed ? sizeof(LaneItem<float>) : sizeof(LaneItem<double>);
     if (c.kind == KIND_TENSOR_LANE) return c.mixed ? sizeof(TensorLaneItem<float>) : sizeof(TensorLaneItem<double>);
     if (c.kind == KIND_LINEAR) return c.mixed ? sizeof(LinearItem<float>) : sizeof(LinearItem<double>);
     if (c.kind == KIND_UMMA) return sizeof(UmmaItem);
@@ -467,6 +514,14 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
         it.block0 = block0;
         it.slot = slot;
         std::memcpy(dst, &it, sizeof(it));
+    } else if (c.kind == KIND_LANE) {
+        LaneItem<KT> it{};
+        for (int par = 0; par < 2; ++par)
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+        it.g = h->lgeo;
+        it.block0 = block0;
+        it.slot = slot;
+        std::memcpy(dst, &it, sizeof(it));
     } else if (c.kind == KIND_TENSOR_LANE) {
         TensorLaneItem<KT> it{};
         for (int par = 0; par < 2; ++par)
@@ -504,6 +559,7 @@ void set_block0(const BatchClass &c, unsigned char *dst, int64_t block0) {
     if (c.kind == KIND_DENSE || c.kind == KIND_WAVE_TILES) put((DenseItem<KT> *)nullptr);
     else if (c.kind == KIND_UMMA) put((UmmaItem *)nullptr);
     else if (c.kind == KIND_LINEAR) put((LinearItem<KT> *)nullptr);
+    else if (c.kind == KIND_LANE) put((LaneItem<KT> *)nullptr);
     else if (c.kind == KIND_TENSOR_LANE) put((TensorLaneItem<KT> *)nullptr);
     else if (c.kind == KIND_TENSOR) put((TensorItem<KT> *)nullptr);
     else put((SliceItem<KT> *)nullptr);
@@ -671,6 +727,52 @@ void launch_grouped_tensor_lane(const hgg_batch *b, const BatchClass &c, int st,
     });
 }
 
+template <typename KT, int DIM, int NFL, int WAVE>
+void launch_grouped_lane(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
+    dense_dispatch<DIM, NFL, WAVE>(c.rep.nB, [&](auto nbc) {
+        constexpr int NB = decltype(nbc)::value;
+        using CT = DenseCT<KT, NB>;
+        if constexpr (lane_size(DIM, NFL, WAVE, NB)) {
+            auto go = [&](auto kern, int threads, int smem) {
+                if (smem > 48 * 1024 - (int)sizeof(LaneItem<KT>))
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                class_kernel(b, kern, grid, threads, smem, s, static_cast<const LaneItem<KT> *>(c.d_items[st]), c.d_n,
+                             c.d_total, b->d_parity, b->d_remaining);
+            };
+            if constexpr (WAVE) {
+                using SH = LaneShape<KT, CT, DIM, NFL, NB, true>;
+                if (st > 0)
+                    go(grouped_wave_lane<KT, CT, CT, DIM, NFL, NB>, SH::THREADS,
+                       wave_lane_smem<KT, CT, CT, DIM, NFL, NB>(c.lane_bytes, SH::TILES));
+                else
+                    go(grouped_wave_lane<KT, CT, double, DIM, NFL, NB>, SH::THREADS,
+                       wave_lane_smem<KT, CT, double, DIM, NFL, NB>(c.lane_bytes, SH::TILES));
+            } else {
+                constexpr int threads = LaneShape<KT, CT, DIM, NFL, NB, false>::THREADS;
+                const int nin = class_nin(c, st);
+                if (nin == 0) go(grouped_advection_lane<KT, CT, DIM, NFL, NB, 0>, threads, c.lane_bytes);
+                else if (nin == 1) go(grouped_advection_lane<KT, CT, DIM, NFL, NB, 1>, threads, c.lane_bytes);
+                else go(grouped_advection_lane<KT, CT, DIM, NFL, NB, -1>, threads, c.lane_bytes);
+            }
+        }
+    });
+}
+
+template <typename KT>
+void launch_grouped_lane_any(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
+    const bool wave = c.physics != HGG_PHYSICS_ADVECTION;
+    switch (c.shape) {
+        case HGG_SHAPE_TRIANGLE:
+            wave ? launch_grouped_lane<KT, 2, 3, 1>(b, c, st, grid, s) : launch_grouped_lane<KT, 2, 3, 0>(b, c, st, grid, s);
+            break;
+        case HGG_SHAPE_TETRAHEDRON:
+            wave ? launch_grouped_lane<KT, 3, 4, 1>(b, c, st, grid, s) : launch_grouped_lane<KT, 3, 4, 0>(b, c, st, grid, s);
+            break;
+        case HGG_SHAPE_SQUARE: launch_grouped_lane<KT, 2, 4, 1>(b, c, st, grid, s); break;
+        case HGG_SHAPE_CUBE: launch_grouped_lane<KT, 3, 6, 1>(b, c, st, grid, s); break;
+    }
+}
+
 template <typename KT>
 void launch_grouped_slice(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
     SliceOps sops;
@@ -786,6 +888,9 @@ void launch_class_stage(hgg_batch *b, const BatchClass &c, int st, cudaStream_t 
                 c.mixed ? launch_grouped_wave<float, 3, 6>(b, c, st, grid, s) : launch_grouped_wave<double, 3, 6>(b, c, st, grid, s);
                 break;
         }
+    } else if (c.kind == KIND_LANE) {
+        if (c.mixed) launch_grouped_lane_any<float>(b, c, st, grid, s);
+        else launch_grouped_lane_any<double>(b, c, st, grid, s);
     } else if (c.kind == KIND_TENSOR_LANE) {
         if (c.mixed) launch_grouped_tensor_lane<float>(b, c, st, grid, s);
         else launch_grouped_tensor_lane<double>(b, c, st, grid, s);
@@ -1148,6 +1253,7 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
         c.precision = h->precision;
         c.rows = h->lin_R;
         c.lslots = h->lin_slots;
+        c.lane_bytes = h->lgeo.group_bytes;
         c.rep.shape = h->op.shape;
         c.rep.dim = h->op.dim;
         c.rep.order = h->op.order;

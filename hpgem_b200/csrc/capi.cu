@@ -54,11 +54,14 @@ int solution_to_host(hgg_handle *h, double *staging, double *out) {
         std::memcpy(out, staging, sizeof(double) * h->N);
         return 0;
     }
-    const int nb = h->op.nB;
+    const int nb = coefficients(h);
     const int64_t ne = h->N / nb;
+    const int32_t *slot = h->slot.empty() ? nullptr : h->slot.data();
     for (int64_t e = 0; e < ne; ++e)
         for (int k = 0; k < nb; ++k)
-            out[e * nb + k] = h->op.tsign[k] * staging[device_index(e, (int)h->op.tpos[k], nb, h->tiled)];
+            out[e * nb + k] = h->op.tensor
+                                  ? h->op.tsign[k] * staging[device_index(e, (int)h->op.tpos[k], nb, h->tiled)]
+                                  : staging[device_index(e, k, nb, h->tiled, slot)];
     return 0;
 }
 
@@ -73,25 +76,28 @@ void release_graphs(hgg_handle *h) {
 // The device vectors of a sum-factorised handle are already in tensor order
 // with the signs folded in, so the kernels see the identity permutation.
 
-// layout conversion kernels (hpGEM order <-> tensor order, signs folded; tiled:
-// 32-element tiles, coefficient-major inside a tile)
+// layout conversion kernels between hpGEM order and the device's: tensor order with the
+// signs folded (tpos null: hpGEM's own order); tiled: 32-element tiles, coefficient-major
+// inside a tile, with the elements in their slots (null: in element order)
 
 template <typename TD>
 __global__ void to_tensor_order(const double *src, TD *dst, const int32_t *tpos, const double *tsign,
-                                int nb, int64_t n, bool tiled) {
+                                int nb, int64_t n, bool tiled, const int32_t *slot) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t e = i / nb;
         const int k = (int)(i - e * nb);
-        dst[device_index(e, tpos[k], nb, tiled)] = (TD)(tsign[k] * src[i]);
+        if (tpos) dst[device_index(e, tpos[k], nb, tiled)] = (TD)(tsign[k] * src[i]);
+        else dst[device_index(e, k, nb, tiled, slot)] = (TD)src[i];
     }
 }
 template <typename TS>
 __global__ void from_tensor_order(const TS *src, double *dst, const int32_t *tpos, const double *tsign,
-                                  int nb, int64_t n, bool tiled) {
+                                  int nb, int64_t n, bool tiled, const int32_t *slot) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t e = i / nb;
         const int k = (int)(i - e * nb);
-        dst[i] = tsign[k] * (double)src[device_index(e, tpos[k], nb, tiled)];
+        dst[i] = tpos ? tsign[k] * (double)src[device_index(e, tpos[k], nb, tiled)]
+                      : (double)src[device_index(e, k, nb, tiled, slot)];
     }
 }
 // zeros the coefficients of the padding elements [n_elements, n_pad) of a device vector
@@ -112,26 +118,28 @@ __global__ void convert_vector(const float *src, double *dst, int64_t n) {
 }
 // a vector from one layout to the other (to tiled or from tiled), element by element
 template <typename T>
-__global__ void relayout(const T *src, T *dst, int nb, int64_t n, bool tiled) {
+__global__ void relayout(const T *src, T *dst, int nb, int64_t n, bool tiled, const int32_t *slot) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t e = i / nb;
         const int k = (int)(i - e * nb);
-        dst[device_index(e, k, nb, tiled)] = src[device_index(e, k, nb, !tiled)];
+        dst[device_index(e, k, nb, tiled, tiled ? slot : nullptr)] = src[device_index(e, k, nb, !tiled, tiled ? nullptr : slot)];
     }
 }
 
 int upload_tensor_geometry(hgg_handle *h);
+int alloc_tile_inputs(hgg_handle *h);
 
 // moves every vector of a handle with a lane kernel between that kernel's layout and the
 // general kernels' (a change of the kernel variant; the padding elements stay zero)
 int set_lane_layout(hgg_handle *h, bool lane) {
     int rc;
-    if (!lane && (rc = upload_tensor_geometry(h))) return rc;
+    if (!lane && h->op.tensor && (rc = upload_tensor_geometry(h))) return rc;
+    if (!lane && h->group_tiles > 0 && (rc = alloc_tile_inputs(h))) return rc;
     auto move = [&](auto *v) {
         using T = std::remove_pointer_t<decltype(v)>;
         T *tmp = reinterpret_cast<T *>(h->d_scratch);
         cudaMemsetAsync(tmp, 0, sizeof(T) * h->N_alloc, h->stream);
-        relayout<T><<<4 * h->num_sms, 256, 0, h->stream>>>(v, tmp, coefficients(h), h->N, lane);
+        relayout<T><<<4 * h->num_sms, 256, 0, h->stream>>>(v, tmp, coefficients(h), h->N, lane, h->d_slot_lane);
         cudaMemcpyAsync(v, tmp, sizeof(T) * h->N_alloc, cudaMemcpyDeviceToDevice, h->stream);
         h->launches++;
     };
@@ -143,12 +151,17 @@ int set_lane_layout(hgg_handle *h, bool lane) {
     HGG_CUDA(h, cudaGetLastError());
     HGG_CUDA(h, cudaStreamSynchronize(h->stream));
     h->lane = h->tiled = lane;
+    if (!h->op.tensor) {
+        h->tensor_layout = lane;
+        h->d_slot = lane ? h->d_slot_lane : nullptr;
+    }
     return 0;
 }
 
 int launch_stage(hgg_handle *h, const StageIO &io) {
     int rc;
-    if (h->linear) rc = launch_stage_linear(h, io);
+    if (h->lane && !h->op.tensor) rc = launch_stage_lane(h, io);
+    else if (h->linear) rc = launch_stage_linear(h, io);
     else if (h->slice_ok || h->op.tensor) rc = launch_stage_tensor(h, io);
     else rc = launch_stage_dense(h, io);
     if (rc) return rc;
@@ -161,7 +174,8 @@ int launch_stage(hgg_handle *h, const StageIO &io) {
 // FP32-mixed form: the stage kernels that have it
 int launch_stage(hgg_handle *h, const StageIOT<float> &io) {
     int rc;
-    if (h->linear) rc = launch_stage_linear(h, io);
+    if (h->lane && !h->op.tensor) rc = launch_stage_lane(h, io);
+    else if (h->linear) rc = launch_stage_linear(h, io);
     else if (h->slice_ok || h->op.tensor) rc = launch_stage_tensor(h, io);
     else rc = launch_stage_dense(h, io);
     if (rc) return rc;
@@ -205,7 +219,7 @@ bool group_wave_wanted(const hgg_handle *h) {
 }
 
 bool forms_next_input(const hgg_handle *h) {
-    if (!h->d_win[0] || h->src || !group_wave_wanted(h)) return false;
+    if (h->lane || !h->d_win[0] || h->src || !group_wave_wanted(h)) return false;
     const int S = h->S;
     for (int i = 1; i < S; ++i)
         for (int j = 0; j < i; ++j)
@@ -353,6 +367,66 @@ int upload_tensor_geometry(hgg_handle *h) {
     return 0;
 }
 
+// stage inputs the tile kernel of the wave forms ahead
+int alloc_tile_inputs(hgg_handle *h) {
+    for (int i = 0; i < 2; ++i)
+        if (int rc = h->d_win[i] ? 0 : alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_win[i])) return rc;
+    return 0;
+}
+
+// Lane kernel of simplices and of the wave: the mesh's groups, their tables (host).
+void lane_setup(hgg_handle *h, LaneMesh &m, LaneTables &t) {
+    const HostOperators &op = h->op;
+    const bool wave = op.physics != HGG_PHYSICS_ADVECTION;
+    if (!lane_size(op.dim, op.nfl, wave, op.nB) || op.nB != lane_basis(op.dim, op.nfl, op.order)) return;
+    // 64-bit handles take the folded tables; the FP32 form keeps its order of operations, and
+    // its folded triangles (p = 5) the stored-matrix tiles
+    const bool folded = !h->mixed;
+    const int elem_bytes = folded || op.nB > kMixedFp32MaxBasis ? 8 : 4;
+    if (h->mixed && !wave && op.shape == HGG_SHAPE_TRIANGLE && op.nB >= 21) return;
+    // a block takes several tiles of a group once every SM has two such blocks: the group's
+    // table is then read from L2 once for all of them
+    const int most = std::max(1, 4 / lane_warps(op.nB, wave ? lane_wave_rows(folded) : kLaneAdvRows));
+    h->lane_tiles = op.nE / 32 >= 2 * (int64_t)most * 148 ? most : 1;
+    const int bytes = 24 + (wave ? 2 * elem_bytes : 0) + h->S * (h->mixed ? 4 : 8);
+    // a server's estimate of a handle's footprint leaves 320 bytes per element and 4 MB, and
+    // the FP32 wave's stage inputs are half of what it counts
+    const int spare = 320 + (wave && elem_bytes == 4 ? 8 * op.V * op.nB : 0);
+    if (!lane_mesh(op, h->lane_tiles, folded, bytes, spare, m)) return;
+    if (!(wave ? lane_wave_tables(op, m, folded, elem_bytes, t)
+                : lane_advection_tables(op, m, folded, elem_bytes, t))) return;
+    if (t.group_bytes > 96 * 1024) return;
+    h->lane_ok = h->lane = h->tensor_layout = true;
+}
+
+int upload_lane(hgg_handle *h, const LaneMesh &m, const LaneTables &t) {
+    int rc;
+    unsigned char *d_tab = nullptr;
+    LaneChunk *d_chunks = nullptr;
+    int32_t *d_nbr = nullptr;
+    double *d_geo = nullptr;
+    if ((rc = upload(h, m.slot, &h->d_slot_lane)) || (rc = upload(h, t.data, &d_tab)) ||
+        (rc = upload(h, m.chunks, &d_chunks)) || (rc = upload(h, m.nbr, &d_nbr)) ||
+        (rc = upload(h, t.geometry, &d_geo)))
+        return rc;
+    if (h->op.physics != HGG_PHYSICS_ADVECTION)
+        for (int i = 0; i < 2; ++i) {
+            if ((rc = alloc(h, (size_t)t.elem_bytes * h->N_alloc, (void **)&h->d_lane_win[i]))) return rc;
+            HGG_CUDA(h, cudaMemsetAsync(h->d_lane_win[i], 0, (size_t)t.elem_bytes * h->N_alloc, h->stream));
+        }
+    h->lgeo.tables = d_tab;
+    h->lgeo.chunks = d_chunks;
+    h->lgeo.geo = d_geo;
+    h->lgeo.nbr = d_nbr;
+    h->lgeo.n_slots = m.n_slots;
+    h->lgeo.n_chunks = (int32_t)m.chunks.size();
+    h->lgeo.group_bytes = (int32_t)t.group_bytes;
+    h->lgeo.column_words = t.column_words;
+    h->slot = m.slot;
+    h->d_slot = h->d_slot_lane;
+    return 0;
+}
+
 // linear: the handle will run the stored-matrix kernel (attach_linear), so the
 // vectors stay in hpGEM order and the matrix-free operators are not uploaded
 int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = false) {
@@ -372,12 +446,15 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
     h->slice_ok = op.tensor && op.dim == 3 && op.order == 3 && op.trace_pos[0] == 0 && op.trace_pos[1] == 1;
     std::vector<int32_t> lane_nbr;
     h->lane_ok = h->lane = !h->slice_ok && tensor_lane_setup(op, h->tlane, lane_nbr);
+    LaneMesh lmesh;
+    LaneTables ltab;
+    if (!op.tensor && !linear && desc->precision != HGG_PRECISION_BF16X3) lane_setup(h, lmesh, ltab);
     h->tiled = h->slice_ok || h->lane;
     if (h->slice_ok) h->tile_elems = SliceShape::TE;
     if (h->mixed && !mixed_supported(h))
         return fail(h, HGG_ERR_UNSUPPORTED, "the FP32-mixed form has no kernel for this shape and order");
     int64_t n_pad = (op.nE + h->tile_elems - 1) / h->tile_elems * h->tile_elems;
-    if (h->lane_ok) n_pad = (n_pad + 31) / 32 * 32;  // whole tiles in either layout
+    if (h->lane_ok) n_pad = std::max((n_pad + 31) / 32 * 32, lmesh.n_slots);  // whole tiles in either layout
     h->N_alloc = n_pad * op.V * op.nB;
     if ((rc = init_device_vectors(h))) return rc;
     if (op.tensor) {
@@ -411,11 +488,12 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
         if ((rc = upload(h, tp, &h->d_tpos)) || (rc = upload(h, op.tsign, &h->d_tsign))) return rc;
         if ((rc = alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_scratch))) return rc;
     } else {
-        if (h->mixed && (rc = alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_scratch))) return rc;
+        if ((h->mixed || h->lane_ok) && (rc = alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_scratch))) return rc;
         if (linear) {
             HGG_CUDA(h, cudaStreamSynchronize(h->stream));
             return 0;
         }
+        if (h->lane_ok && (rc = upload_lane(h, lmesh, ltab))) return rc;
         // Folded operator: for advection on triangles of order >= 4 (>= 5 in the
         // mixed form) the element's whole stage is one small dense operator per
         // matrix slot (the reference's integrands assembled once, the mass inverse
@@ -510,9 +588,10 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
             if (n_tiles * TE <= 2 * op.nE) {
                 if ((rc = upload(h, tiles, &h->d_group_tiles))) return rc;
                 h->group_tiles = n_tiles;
-                for (int i = 0; i < 2; ++i)
-                    if ((rc = alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_win[i]))) return rc;
+                if (!h->lane_ok && (rc = alloc_tile_inputs(h))) return rc;
             }
+            // (before any change of the variant: the kernel the lane kernel stands in for)
+            h->lgeo.neighbour_fp64 = group_wave_wanted(h);
         }
         if ((rc = upload(h, transposed(op.vol), &h->d_vol)) || (rc = upload(h, transposed(op.pairs), &h->d_pairs)) ||
             (rc = upload(h, op.nbr, &h->d_nbr)) || (rc = upload(h, op.self_pair, &h->d_self)) ||
@@ -715,10 +794,10 @@ int hgg_set_state(hgg_handle *h, int32_t vec, const double *host) {
         HGG_CUDA(h, cudaMemcpyAsync(h->d_scratch, host, sizeof(double) * h->N, cudaMemcpyHostToDevice, h->stream));
         if (h->tensor_layout && f)
             to_tensor_order<float><<<grid, 256, 0, h->stream>>>(h->d_scratch, static_cast<float *>(d), h->d_tpos,
-                                                                 h->d_tsign, h->op.nB, h->N, h->tiled);
+                                                                 h->d_tsign, coefficients(h), h->N, h->tiled, h->d_slot);
         else if (h->tensor_layout)
             to_tensor_order<double><<<grid, 256, 0, h->stream>>>(h->d_scratch, static_cast<double *>(d), h->d_tpos,
-                                                                  h->d_tsign, h->op.nB, h->N, h->tiled);
+                                                                  h->d_tsign, coefficients(h), h->N, h->tiled, h->d_slot);
         else
             convert_vector<<<grid, 256, 0, h->stream>>>(h->d_scratch, static_cast<float *>(d), h->N);
         h->launches++;
@@ -740,10 +819,10 @@ int hgg_get_state(hgg_handle *h, int32_t vec, double *host) {
     if (h->tensor_layout || f) {
         if (h->tensor_layout && f)
             from_tensor_order<float><<<grid, 256, 0, h->stream>>>(static_cast<const float *>(d), h->d_scratch,
-                                                                   h->d_tpos, h->d_tsign, h->op.nB, h->N, h->tiled);
+                                                                   h->d_tpos, h->d_tsign, coefficients(h), h->N, h->tiled, h->d_slot);
         else if (h->tensor_layout)
             from_tensor_order<double><<<grid, 256, 0, h->stream>>>(static_cast<const double *>(d), h->d_scratch,
-                                                                    h->d_tpos, h->d_tsign, h->op.nB, h->N, h->tiled);
+                                                                    h->d_tpos, h->d_tsign, coefficients(h), h->N, h->tiled, h->d_slot);
         else
             convert_vector<<<grid, 256, 0, h->stream>>>(static_cast<const float *>(d), h->d_scratch, h->N);
         h->launches++;
@@ -915,10 +994,13 @@ int hgg_time_derivative_static(hgg_handle *h, const double *u, double *k) {
     StageIO io{};
     io.n_elements = h->op.nE;
     io.status = h->d_status;
-    if (!h->tensor_layout) {  // the dense kernels read and write hpGEM order: no scratch
+    if (!h->op.tensor) {  // the general dense kernels read and write hpGEM order: no scratch
         io.u = u;
         io.kout = k;
+        const bool lane = h->lane;
+        h->lane = false;
         int rc = launch_stage(h, io);
+        h->lane = lane;
         if (rc) return rc;
         return check_status(h);
     }
@@ -954,16 +1036,16 @@ int hgg_time_derivative_static(hgg_handle *h, const double *u, double *k) {
             su, nbv, h->op.nE, n_pad, h->tiled);
         h->launches++;
     }
-    to_tensor_order<double><<<4 * h->num_sms, 256, 0, h->stream>>>(u, su, h->d_tpos, h->d_tsign, h->op.nB, h->N,
-                                                                    h->tiled);
+    to_tensor_order<double><<<4 * h->num_sms, 256, 0, h->stream>>>(u, su, h->d_tpos, h->d_tsign, coefficients(h), h->N,
+                                                                    h->tiled, h->d_slot);
     h->launches++;
     HGG_CUDA(h, cudaGetLastError());
     io.u = su;
     io.kout = sk;
     int rc = launch_stage(h, io);
     if (rc) return rc;
-    from_tensor_order<double><<<4 * h->num_sms, 256, 0, h->stream>>>(sk, k, h->d_tpos, h->d_tsign, h->op.nB, h->N,
-                                                                      h->tiled);
+    from_tensor_order<double><<<4 * h->num_sms, 256, 0, h->stream>>>(sk, k, h->d_tpos, h->d_tsign, coefficients(h), h->N,
+                                                                      h->tiled, h->d_slot);
     h->launches++;
     HGG_CUDA(h, cudaGetLastError());
     return check_status(h);
@@ -979,12 +1061,12 @@ int hgg_time_derivative_static(hgg_handle *h, const double *u, double *k) {
 // sign flips inside each element, which leaves both norms unchanged.
 template <typename KT>
 __global__ void element_error_norm(const double *u, ErrStages<KT> ks, int nb, int64_t n_elements, bool tiled,
-                                   double *err2, double *norm) {
+                                   const int32_t *slot, double *err2, double *norm) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= n_elements) return;
     double s2 = 0.0, n2 = 0.0;
     for (int pos = 0; pos < nb; ++pos) {
-        const int64_t idx = device_index(e, pos, nb, tiled);
+        const int64_t idx = device_index(e, pos, nb, tiled, slot);
         double dev = 0.0;
         for (int i = 0; i < ks.n; ++i) dev += ((double)ks.k[i][idx] * ks.dt) * ks.err[i];
         s2 += dev * dev;
@@ -1052,10 +1134,10 @@ int error_and_norm(hgg_handle *h, double dt, double *error, double *norm) {
     const unsigned eb = (unsigned)((nE + 255) / 256);
     if (h->mixed)
         element_error_norm<float><<<eb, 256, 0, h->stream>>>(h->sol[h->cur], err_stages<float>(h, dt, h->rk_err), nb,
-                                                             nE, h->tiled, err2, nrm);
+                                                             nE, h->tiled, h->d_slot, err2, nrm);
     else
         element_error_norm<double><<<eb, 256, 0, h->stream>>>(h->sol[h->cur], err_stages<double>(h, dt, h->rk_err),
-                                                              nb, nE, h->tiled, err2, nrm);
+                                                              nb, nE, h->tiled, h->d_slot, err2, nrm);
     const int parts = 256;
     double *pa = h->d_reduce + 2 * nE, *pb = pa + parts;
     sum_pairs<<<parts, kSumThreads, 0, h->stream>>>(err2, nrm, nE, pa, pb);
@@ -1561,10 +1643,10 @@ int hpgem_order_view(hgg_handle *h, int vec, const double **view) {
     const unsigned grid = 4 * h->num_sms;
     if (h->tensor_layout && f)
         from_tensor_order<float><<<grid, 256, 0, h->stream>>>(static_cast<const float *>(d), h->d_scratch, h->d_tpos,
-                                                               h->d_tsign, h->op.nB, h->N, h->tiled);
+                                                               h->d_tsign, coefficients(h), h->N, h->tiled, h->d_slot);
     else if (h->tensor_layout)
         from_tensor_order<double><<<grid, 256, 0, h->stream>>>(static_cast<const double *>(d), h->d_scratch,
-                                                                h->d_tpos, h->d_tsign, h->op.nB, h->N, h->tiled);
+                                                                h->d_tpos, h->d_tsign, coefficients(h), h->N, h->tiled, h->d_slot);
     else
         convert_vector<<<grid, 256, 0, h->stream>>>(static_cast<const float *>(d), h->d_scratch, h->N);
     h->launches++;

@@ -12,6 +12,7 @@
 
 #include "../../include/hpgem_b200.h"
 #include "dg_kernels.cuh"
+#include "lane_stage.cuh"
 #include "linear_stage.cuh"
 #include "linear_umma.cuh"
 #include "tensor_lane.cuh"
@@ -73,7 +74,13 @@ struct hgg_handle {
     // one-element-per-thread kernels (lane = element, tiled layout): the handle has one, and
     // its vectors are in that kernel's layout (kernel variant 0)
     bool lane_ok = false, lane = false;
-    hgg::TensorLaneGeom tlane{};
+    hgg::TensorLaneGeom tlane{};          // sum-factorised handles
+    hgg::LaneGeom lgeo{};                  // simplices and the wave
+    double *d_lane_win[2] = {nullptr, nullptr};  // ... the wave: stage inputs formed ahead (contraction type)
+    int lane_tiles = 1;                    // ... tiles of a chunk at most
+    std::vector<int32_t> slot;            // place of each element in the lane layout (empty: its own number)
+    int32_t *d_slot = nullptr;            // slot on the device while the lane layout is in use, else null
+    int32_t *d_slot_lane = nullptr;
     // stored-matrix form (HpgemAPILinear): distinct folded matrices, transposed
     bool linear = false;
     int lin_R = 0, lin_slots = 0, lin_mats = 0;
@@ -176,7 +183,10 @@ TensorConsts<P, DIM> tensor_consts(const HostOperators &op) {
 
 // layout conversion index (hpGEM order <-> tensor order, signs folded; tiled:
 // 32-element tiles, coefficient-major inside a tile)
-__host__ __device__ __forceinline__ int64_t device_index(int64_t e, int pos, int nb, bool tiled) {
+// slot: the place of each element in the tiles, or null for its own number
+__host__ __device__ __forceinline__ int64_t device_index(int64_t e, int pos, int nb, bool tiled,
+                                                         const int32_t *slot = nullptr) {
+    if (slot) e = slot[e];
     return tiled ? (e >> 5) * ((int64_t)nb << 5) + (int64_t)pos * 32 + (e & 31) : e * nb + pos;
 }
 // stage vectors and per-stage coefficients of the error estimate and the rewind
@@ -200,6 +210,8 @@ int launch_stage_tensor(hgg_handle *h, const StageIOT<double> &io);
 int launch_stage_tensor(hgg_handle *h, const StageIOT<float> &io);
 int launch_stage_dense(hgg_handle *h, const StageIOT<double> &io);
 int launch_stage_dense(hgg_handle *h, const StageIOT<float> &io);
+int launch_stage_lane(hgg_handle *h, const StageIOT<double> &io);
+int launch_stage_lane(hgg_handle *h, const StageIOT<float> &io);
 int launch_stage_linear(hgg_handle *h, const StageIOT<double> &io);
 int launch_stage_linear(hgg_handle *h, const StageIOT<float> &io);
 // the handle's stage kernel, counted, with the launch error checked
@@ -208,6 +220,11 @@ int launch_stage(hgg_handle *h, const StageIOT<float> &io);
 
 void *vector_ptr(hgg_handle *h, int vec);
 bool vector_is_float(const hgg_handle *h, int vec);
+
+// the wave's lane kernel reads one vector: every stage but the last forms the next one's input
+inline bool lane_forms_input(const hgg_handle *h) {
+    return h->lane && !h->op.tensor && h->op.physics != HGG_PHYSICS_ADVECTION;
+}
 
 // Inputs and outputs of stage i of one Runge-Kutta step from sol[from] into
 // sol[1 - from] (stages as in HpgemAPISimplified_Impl.h:788-820; zero tableau
@@ -241,6 +258,21 @@ StageIOT<KT> make_stage_io(const hgg_handle *h, int from, double dt, int i, int 
             }
         }
         io.blast = dt * h->rk_b[S - 1];
+    }
+    if (lane_forms_input(h)) {
+        if (i > 0) io.win = h->d_lane_win[(i - 1) & 1];
+        if (!last) {
+            io.wnext = h->d_lane_win[i & 1];
+            for (int j = 0; j < i; ++j) {
+                const double c = dt * h->rk_a[(i + 1) * S + j];
+                if (c != 0.0) {
+                    io.kfin[io.nfin] = kv(j);
+                    io.bfin[io.nfin] = c;
+                    io.nfin++;
+                }
+            }
+            io.wcoef = dt * h->rk_a[(i + 1) * S + i];
+        }
     }
     return io;
 }

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 namespace hgg {
 
@@ -59,6 +60,341 @@ bool tensor_lane_setup(const HostOperators &op, TensorLaneGeom &g, std::vector<i
     for (int64_t e = 0; e < op.nE; ++e)
         for (int c = 0; c < d; ++c)
             if (g.side[c] >= 0) nbr[((e >> 5) * d + c) * 32 + (e & 31)] = op.t_nbr[e * ns + 2 * c + g.side[c]];
+    return true;
+}
+
+// ---- simplices and the wave -------------------------------------------------------
+
+namespace {
+
+// The first pair operator equal to each one.  A face's points are numbered from its left
+// element, so one operator appears once per numbering; the copies differ by rounding.
+std::vector<int32_t> same_pairs(const HostOperators &op) {
+    const size_t nn = (size_t)op.nB * op.nB;
+    std::vector<int32_t> same(op.n_pairs);
+    for (int p = 0; p < op.n_pairs; ++p) {
+        const double *A = &op.pairs[p * nn];
+        double big = 0.0;
+        for (size_t i = 0; i < nn; ++i) big = std::max(big, std::fabs(A[i]));
+        same[p] = p;
+        for (int q = 0; q < p && same[p] == p; ++q) {
+            if (same[q] != q) continue;
+            const double *B = &op.pairs[q * nn];
+            bool eq = std::equal(&op.pair_trace[(size_t)p * op.nB], &op.pair_trace[(size_t)(p + 1) * op.nB],
+                                 &op.pair_trace[(size_t)q * op.nB]);
+            for (size_t i = 0; i < nn && eq; ++i) eq = std::fabs(A[i] - B[i]) <= 0x1p-40 * big;
+            if (eq) same[p] = q;
+        }
+    }
+    return same;
+}
+
+}  // namespace
+
+bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int coefficient_bytes, int spare_bytes, LaneMesh &m) {
+    const int nf = op.nfl, d = op.dim, R = op.V * op.nB;
+    const bool wave = op.physics != 0;
+    // (plain tables hold no geometry: their kernels read every element's own)
+    const int eg = !folded ? 0 : wave ? d * d : d, fg = !folded ? 0 : wave ? d : 1;
+    // group key: pair operators, upwind modes, and the geometry rounded to 2^-40 of its
+    // largest entry (only the key is rounded; a group steps with its first element's
+    // values, which differ from the others' by the rounding of vertex coordinates).
+    // (the plain tables' results depend on their operators' last bits: no merging there)
+    std::vector<int32_t> same;
+    if (folded) same = same_pairs(op);
+    else
+        for (int p = 0; p < op.n_pairs; ++p) same.push_back(p);
+    m = LaneMesh{};
+    std::vector<int32_t> group(op.nE);
+    std::vector<int64_t> count;
+    const int words = 2 * nf + eg + nf * fg + 2;
+    std::vector<uint64_t> key(words), keys;  // of one element, of the groups
+    std::vector<int32_t> table(1024, -1);    // open addressing: groups by hash
+    auto put = [&](uint64_t *dst, const double *v, int n) {
+        double big = 0.0;
+        for (int i = 0; i < n; ++i) big = std::max(big, std::fabs(v[i]));
+        if (!std::isfinite(big)) return false;
+        int e = 0;
+        std::frexp(big, &e);
+        // adding 1.5 * 2^52 rounds to a whole number (the scaled values are below 2^40)
+        const double scale = big > 0.0 ? std::ldexp(1.0, 40 - e) : 0.0, magic = 0x1.8p52;
+        for (int i = 0; i < n; ++i) {
+            const volatile double r = v[i] * scale + magic;
+            const double q = r;
+            std::memcpy(&dst[i], &q, sizeof(q));
+        }
+        dst[n] = (uint64_t)(int64_t)e;
+        return true;
+    };
+    const size_t most = (size_t)op.nE / 16 + 64;  // more groups than this cannot fill tiles
+    for (int64_t e = 0; e < op.nE; ++e) {
+        uint64_t *k = key.data();
+        for (int f = 0; f < nf; ++f) {
+            *k++ = (uint64_t)(uint32_t)same[op.self_pair[e * nf + f]] << 32 | (uint32_t)same[op.nbr_pair[e * nf + f]];
+            *k++ = (uint64_t)op.mode[e * nf + f];
+        }
+        if (!put(k, &op.elem_geo[e * eg], eg) || !put(k + eg + 1, &op.face_geo[e * nf * fg], nf * fg)) return false;
+        uint64_t hash = 0;
+        for (uint64_t w : key) {
+            hash = (hash ^ w) * 0x9E3779B97F4A7C15ull;
+            hash ^= hash >> 29;
+        }
+        size_t at = hash & (table.size() - 1);
+        while (table[at] >= 0 && !std::equal(key.begin(), key.end(), keys.begin() + (size_t)table[at] * words))
+            at = (at + 1) & (table.size() - 1);
+        if (table[at] < 0) {
+            if (count.size() >= most || count.size() * 2 >= table.size()) return false;
+            table[at] = (int32_t)count.size();
+            keys.insert(keys.end(), key.begin(), key.end());
+            m.representative.push_back(e);
+            count.push_back(0);
+        }
+        group[e] = table[at];
+        count[group[e]]++;
+    }
+    int64_t tiles = 0;
+    for (int64_t c : count) tiles += (c + 31) / 32;
+    const int64_t pad = tiles * 32 - op.nE;
+    // padded slots cost idle lanes and memory in every vector: at most half as many as
+    // elements (or two tiles), and within spare_bytes per element and 4 MB
+    if (pad > std::max<int64_t>(op.nE / 2, 64)) return false;
+    if ((double)pad * R * coefficient_bytes > (double)spare_bytes * (double)op.nE + 4e6) return false;
+    if (tiles > INT32_MAX / 32) return false;
+    m.n_slots = tiles * 32;
+    // chunks of a group in element order, then all chunks by their first element, so that
+    // neighbours in other groups run at about the same time
+    const int per = 32 * chunk_tiles_max;
+    std::vector<std::vector<int64_t>> members(count.size());
+    for (size_t g = 0; g < count.size(); ++g) members[g].reserve(count[g]);
+    for (int64_t e = 0; e < op.nE; ++e) members[group[e]].push_back(e);
+    struct Piece {
+        int64_t first;
+        int32_t group;
+        int64_t at;
+    };
+    std::vector<Piece> pieces;
+    for (size_t g = 0; g < members.size(); ++g)
+        for (int64_t at = 0; at < count[g]; at += per) pieces.push_back({members[g][at], (int32_t)g, at});
+    std::sort(pieces.begin(), pieces.end(), [](const Piece &a, const Piece &b) { return a.first < b.first; });
+    m.slot.assign(op.nE, 0);
+    int32_t tile = 0;
+    for (const Piece &p : pieces) {
+        const int64_t n = std::min<int64_t>(per, count[p.group] - p.at);
+        const int32_t nt = (int32_t)((n + 31) / 32);
+        m.chunks.push_back({tile, nt, p.group, 0});
+        for (int64_t i = 0; i < n; ++i) m.slot[members[p.group][p.at + i]] = tile * 32 + (int32_t)i;
+        tile += nt;
+    }
+    m.nbr.assign((size_t)tiles * nf * 32, 0);
+    for (int64_t e = 0; e < op.nE; ++e)
+        for (int f = 0; f < nf; ++f)
+            m.nbr[((size_t)(m.slot[e] >> 5) * nf + f) * 32 + (m.slot[e] & 31)] = m.slot[op.nbr[e * nf + f]];
+    return true;
+}
+
+namespace {
+
+// functions of a face operator's trial side that do not vanish on the face; false when
+// there are more than `most`
+bool trace_columns(const HostOperators &op, int32_t pair, int most, std::vector<int32_t> &cols) {
+    cols.clear();
+    for (int j = 0; j < op.nB; ++j)
+        if (op.pair_trace[(size_t)pair * op.nB + j]) cols.push_back(j);
+    return (int)cols.size() <= most;
+}
+
+// appends to a group's table
+struct Writer {
+    std::vector<unsigned char> bytes;
+    template <typename T>
+    void put(T v) {
+        const unsigned char *p = reinterpret_cast<const unsigned char *>(&v);
+        bytes.insert(bytes.end(), p, p + sizeof(T));
+    }
+    // a value, or a column, of the contraction type
+    void number(int elem_bytes, double v) {
+        if (elem_bytes == 8) put(v);
+        else put((float)v);
+    }
+    void plain_column(int elem_bytes, const double *A, int nb, int j, int r0, int rb, int rbp) {
+        if (elem_bytes == 8) column<double>(A, nb, j, r0, rb, rbp, 1.0);
+        else column<float>(A, nb, j, r0, rb, rbp, 1.0);
+    }
+    // column j of A ([nb][nb], scaled): rows r0 .. r0 + rb, padded with zeros
+    template <typename T>
+    void column(const double *A, int nb, int j, int r0, int rb, int rbp, double scale) {
+        for (int i = 0; i < rbp; ++i)
+            put((T)(i < rb && r0 + i < nb && A ? scale * A[(size_t)(r0 + i) * nb + j] : 0.0));
+    }
+};
+
+// pads the group's table to 16 bytes, `tail` (a whole number of words) at its end
+void finish_group(LaneTables &t, Writer &w, const std::vector<int32_t> &tail = {}) {
+    while ((w.bytes.size() + 4 * tail.size()) % 16) w.put((unsigned char)0);
+    for (int32_t v : tail) w.put(v);
+    t.column_words = (int)tail.size();
+    if (t.group_bytes && t.group_bytes != w.bytes.size()) w.bytes.resize(t.group_bytes, 0);
+    t.group_bytes = w.bytes.size();
+    t.data.insert(t.data.end(), w.bytes.begin(), w.bytes.end());
+}
+
+// every element's geometry in its slot: [tile][element's values, faces' values][32]
+void lane_geometry(const HostOperators &op, const LaneMesh &m, std::vector<double> &geo) {
+    const size_t eg = op.elem_geo.size() / op.nE, fg = op.face_geo.size() / op.nE, q = eg + fg;
+    geo.assign((size_t)m.n_slots * q, 0.0);
+    for (int64_t e = 0; e < op.nE; ++e) {
+        double *g = &geo[(size_t)(m.slot[e] >> 5) * q * 32 + (m.slot[e] & 31)];
+        for (size_t i = 0; i < eg; ++i) g[32 * i] = op.elem_geo[e * eg + i];
+        for (size_t i = 0; i < fg; ++i) g[32 * (eg + i)] = op.face_geo[e * fg + i];
+    }
+}
+
+}  // namespace
+
+bool lane_wave_tables(const HostOperators &op, const LaneMesh &m, bool folded, int elem_bytes, LaneTables &t) {
+    const int nb = op.nB, d = op.dim, nf = op.nfl, nfc = lane_trace(d, nf, op.order);
+    const size_t nn = (size_t)nb * nb;
+    const int most = lane_wave_rows(folded);
+    const int rw = lane_warps(nb, most), rb = lane_rows(nb, most);
+    const double invc = 1.0 / op.c_inv;
+    const double c = op.physics == HGG_PHYSICS_WAVE_UPWIND ? 1.0 / std::sqrt(op.c_inv) : 0.0;
+    t = LaneTables{};
+    t.folded = folded;
+    t.elem_bytes = elem_bytes;
+    if (!folded) lane_geometry(op, m, t.geometry);
+    for (int64_t e : m.representative) {
+        const double *G = &op.elem_geo[e * d * d];  // G[dir][c]
+        Writer w;
+        // trace functions of both sides of every face: [face][own, neighbour][nfc], -1 past the last
+        std::vector<int32_t> cs, cn, columns, neighbour_columns;
+        for (int f = 0; f < nf && folded; ++f) {
+            if (!trace_columns(op, op.self_pair[e * nf + f], nfc, cs) ||
+                !trace_columns(op, op.nbr_pair[e * nf + f], nfc, cn))
+                return false;
+            for (auto *v : {&cs, &cn}) {
+                const size_t have = v->size();
+                for (int i = 0; i < nfc; ++i) columns.push_back(i < (int)have ? (*v)[i] : -1);
+            }
+            for (int i = 0; i < nfc; ++i) neighbour_columns.push_back(32 * std::max(columns[(2 * f + 1) * nfc + i], 0));
+        }
+        if (folded) {
+            // physical derivatives D_dir = sum_c G[dir][c] vol_c
+            std::vector<double> D(d * nn, 0.0);
+            for (int a = 0; a < d; ++a)
+                for (int k = 0; k < d; ++k)
+                    for (size_t i = 0; i < nn; ++i) D[a * nn + i] += G[a * d + k] * op.vol[k * nn + i];
+            const int rbp = lane_pad(rb, 8);
+            for (int r = 0; r < rw; ++r) {
+                for (int j = 0; j < nb; ++j)
+                    for (int a = 0; a < d; ++a) w.column<double>(&D[a * nn], nb, j, r * rb, rb, rbp, 1.0);
+                for (int f = 0; f < nf; ++f) {
+                    const double *S = &op.pairs[op.self_pair[e * nf + f] * nn];
+                    const double *N = &op.pairs[op.nbr_pair[e * nf + f] * nn];
+                    for (int i = 0; i < nfc; ++i) {
+                        const int js = columns[(f * 2) * nfc + i], jn = columns[(f * 2 + 1) * nfc + i];
+                        w.column<double>(js >= 0 ? S : nullptr, nb, js, r * rb, rb, rbp, 1.0);
+                        w.column<double>(jn >= 0 ? N : nullptr, nb, jn, r * rb, rb, rbp, 1.0);
+                    }
+                }
+            }
+            for (int f = 0; f < nf; ++f) {
+                const double *nu = &op.face_geo[(e * nf + f) * d];
+                double q = 0.0;
+                for (int a = 0; a < d; ++a) q += nu[a] * nu[a];
+                const double len = std::sqrt(q);
+                for (int a = 0; a < d; ++a) w.put(nu[a]);
+                w.put(c * len);
+                for (int a = 0; a < d; ++a) w.put(invc * nu[a]);
+                for (int a = 0; a < d; ++a) w.put(c == 0.0 ? 0.0 : c * (nu[a] / len));
+            }
+            w.put(invc);
+            for (int f = 0; f < nf; ++f)
+                for (int i = 0; i < nfc; ++i) w.put((int32_t)(32 * std::max(columns[2 * f * nfc + i], 0)));
+        } else {
+            const int rbp = lane_pad(rb, elem_bytes);
+            for (int r = 0; r < rw; ++r) {
+                for (int j = 0; j < nb; ++j)
+                    for (int a = 0; a < d; ++a) w.plain_column(elem_bytes, &op.vol[a * nn], nb, j, r * rb, rb, rbp);
+                for (int f = 0; f < nf; ++f)
+                    for (int j = 0; j < nb; ++j) {
+                        w.plain_column(elem_bytes, &op.pairs[op.self_pair[e * nf + f] * nn], nb, j, r * rb, rb, rbp);
+                        w.plain_column(elem_bytes, &op.pairs[op.nbr_pair[e * nf + f] * nn], nb, j, r * rb, rb, rbp);
+                    }
+            }
+            w.number(elem_bytes, c);
+            w.number(elem_bytes, invc);
+        }
+        finish_group(t, w, neighbour_columns);
+    }
+    return true;
+}
+
+bool lane_advection_tables(const HostOperators &op, const LaneMesh &m, bool folded, int elem_bytes, LaneTables &t) {
+    const int nb = op.nB, d = op.dim, nf = op.nfl, nfc = lane_trace(d, nf, op.order);
+    const size_t nn = (size_t)nb * nb;
+    const int rw = lane_warps(nb, kLaneAdvRows), rb = lane_rows(nb, kLaneAdvRows);
+    t = LaneTables{};
+    t.folded = folded;
+    t.elem_bytes = elem_bytes;
+    if (!folded) {  // a face along the flow has no flux (the plain kernel has no average)
+        for (size_t i = 0; i < op.mode.size(); ++i)
+            if (op.mode[i] == MODE_AVG && op.face_geo[i] != 0.0) return false;
+        lane_geometry(op, m, t.geometry);
+    }
+    for (int64_t e : m.representative) {
+        const double *ahat = &op.elem_geo[e * d], *sigma = &op.face_geo[e * nf];
+        const int8_t *mode = &op.mode[e * nf];
+        Writer w;
+        if (folded) {
+            // own matrix: volume and the faces the element's own trace leaves through
+            std::vector<double> A(nn, 0.0);
+            std::vector<int32_t> faces, columns, cols;
+            std::vector<double> weight;
+            for (int k = 0; k < d; ++k)
+                for (size_t i = 0; i < nn; ++i) A[i] += ahat[k] * op.vol[k * nn + i];
+            for (int f = 0; f < nf; ++f) {
+                if (mode[f] == MODE_NONE || sigma[f] == 0.0) continue;
+                const double s = mode[f] == MODE_AVG ? 0.5 * sigma[f] : sigma[f];
+                if (mode[f] != MODE_NBR) {
+                    const double *S = &op.pairs[op.self_pair[e * nf + f] * nn];
+                    for (size_t i = 0; i < nn; ++i) A[i] -= s * S[i];
+                }
+                if (mode[f] != MODE_SELF) {
+                    if (!trace_columns(op, op.nbr_pair[e * nf + f], nfc, cols)) return false;
+                    faces.push_back(f);
+                    weight.push_back(-s);
+                    const size_t have = cols.size();
+                    for (int i = 0; i < nfc; ++i) columns.push_back(i < (int)have ? cols[i] : -1);
+                }
+            }
+            const int rbp = lane_pad(rb, 8);
+            for (int r = 0; r < rw; ++r) {
+                for (int j = 0; j < nb; ++j) w.column<double>(A.data(), nb, j, r * rb, rb, rbp, 1.0);
+                for (int k = 0; k < nf; ++k)
+                    for (int i = 0; i < nfc; ++i) {
+                        const int j = k < (int)faces.size() ? columns[k * nfc + i] : -1;
+                        const double *N = j >= 0 ? &op.pairs[op.nbr_pair[e * nf + faces[k]] * nn] : nullptr;
+                        w.column<double>(N, nb, j, r * rb, rb, rbp, j >= 0 ? weight[k] : 0.0);
+                    }
+            }
+            w.put((int32_t)faces.size());
+            for (int k = 0; k < nf; ++k) w.put((int32_t)(k < (int)faces.size() ? faces[k] : 0));
+            for (int k = 0; k < nf * nfc; ++k)
+                w.put((int32_t)(k < (int)columns.size() ? 32 * std::max(columns[k], 0) : 0));
+        } else {
+            const int rbp = lane_pad(rb, elem_bytes);
+            for (int r = 0; r < rw; ++r) {
+                for (int j = 0; j < nb; ++j)
+                    for (int a = 0; a < d; ++a) w.plain_column(elem_bytes, &op.vol[a * nn], nb, j, r * rb, rb, rbp);
+                for (int f = 0; f < nf; ++f) {
+                    const int32_t pair = mode[f] == MODE_SELF ? op.self_pair[e * nf + f] : op.nbr_pair[e * nf + f];
+                    for (int j = 0; j < nb; ++j) w.plain_column(elem_bytes, &op.pairs[pair * nn], nb, j, r * rb, rb, rbp);
+                }
+            }
+            for (int f = 0; f < nf; ++f) w.put((int32_t)(mode[f] == MODE_AVG ? MODE_NONE : mode[f]));
+        }
+        finish_group(t, w);
+    }
     return true;
 }
 

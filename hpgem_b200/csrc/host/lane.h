@@ -2,10 +2,17 @@
 // they take and the operators their threads share.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
 #include "operators.h"
+
+#ifdef __CUDACC__
+#define HGG_HOST_DEVICE __host__ __device__
+#else
+#define HGG_HOST_DEVICE
+#endif
 
 namespace hgg {
 
@@ -33,5 +40,66 @@ inline bool tensor_lane_order(int dim, int p) { return (dim == 2 && p >= 1 && p 
 // to 2^-40 of the largest entry (the cells of a structured mesh differ by the rounding of
 // their vertex coordinates; all of them then step with the first element's values).
 bool tensor_lane_setup(const HostOperators &op, TensorLaneGeom &g, std::vector<int32_t> &nbr);
+
+// ---- simplices and the wave (lane_stage.cuh) -------------------------------------
+// Elements with the same operators and geometry (a few groups on a structured mesh) are
+// stored together: tiles of 32 elements of one group, up to `chunk_tiles` tiles of a group
+// in a chunk, which is one block's work.  slot[e] = 32 tile + lane is element e's place.
+struct LaneChunk {
+    int32_t tile0, tiles, group, pad;
+};
+struct LaneMesh {
+    int64_t n_slots = 0;
+    std::vector<int32_t> slot;         // [E]
+    std::vector<int32_t> nbr;          // [tile][nfl][32] the neighbours' slots (padding: 0)
+    std::vector<LaneChunk> chunks;
+    std::vector<int64_t> representative;  // [group] its first element
+};
+
+// rows of an element's output one thread forms (all variables): the element's nb basis
+// rows are split evenly over the fewest warps of at most max_rows rows
+HGG_HOST_DEVICE constexpr int lane_warps(int nb, int max_rows) { return (nb + max_rows - 1) / max_rows; }
+HGG_HOST_DEVICE constexpr int lane_rows(int nb, int max_rows) {
+    return (nb + lane_warps(nb, max_rows) - 1) / lane_warps(nb, max_rows);
+}
+// the wave: four fields per row, so ten rows are 40 64-bit accumulators; the FP32 form
+// keeps every face's two sums as well
+HGG_HOST_DEVICE constexpr int lane_wave_rows(bool folded) { return folded ? 10 : 6; }
+constexpr int kLaneAdvRows = 28;    // one field per row
+// operator rows are padded to 16 bytes
+HGG_HOST_DEVICE constexpr int lane_pad(int rows, int elem_bytes) { return elem_bytes == 8 ? (rows + 1) & ~1 : (rows + 3) & ~3; }
+// basis functions that do not vanish on a face: the trace space of order p
+HGG_HOST_DEVICE constexpr int lane_trace(int dim, int nfl, int p) {
+    return dim == 2 ? p + 1 : (nfl == 4 ? (p + 1) * (p + 2) / 2 : (p + 1) * (p + 1));
+}
+
+// functions of the complete basis of order p
+HGG_HOST_DEVICE constexpr int lane_basis(int dim, int nfl, int p) {
+    return nfl == dim + 1 ? (dim == 2 ? (p + 1) * (p + 2) / 2 : (p + 1) * (p + 2) * (p + 3) / 6)
+                          : (dim == 2 ? (p + 1) * (p + 1) : (p + 1) * (p + 1) * (p + 1));
+}
+
+// What a thread block reads of its group.  The sizes are in elements of the contraction
+// type (8 bytes folded, 4 bytes in the FP32 form).
+struct LaneTables {
+    bool folded = true;              // folded geometry (64-bit handles), else as the FP32 form computes
+    int elem_bytes = 8;              // contraction type
+    size_t group_bytes = 0;          // bytes of one group's table, a multiple of 16
+    int column_words = 0;            // the wave: words of the neighbours' column lists at its end
+    std::vector<unsigned char> data;  // [group][group_bytes]
+    std::vector<double> geometry;    // plain tables: every element's, [tile][Q][32]
+};
+
+// Groups the elements; false when whole tiles of them would take too much padding
+// (unstructured meshes, very small ones).
+// coefficient_bytes: of all vectors of the handle, per coefficient; spare_bytes: what the
+// padding may take per element (and 4 MB).
+bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int coefficient_bytes, int spare_bytes, LaneMesh &m);
+// Tables of the groups: `folded` as described in lane_stage.cuh, or plain with entries of
+// elem_bytes; false when the operators
+// do not have the sparsity it relies on (a face couples more functions than its trace
+// space has) or a flux form it does not take.
+bool lane_wave_tables(const HostOperators &op, const LaneMesh &m, bool folded, int elem_bytes, LaneTables &t);
+bool lane_advection_tables(const HostOperators &op, const LaneMesh &m, bool folded, int elem_bytes, LaneTables &t);
 
 }  // namespace hgg

@@ -370,6 +370,14 @@ HostOperators build_operators(const hgg_problem_desc &desc, bool faces) {
         for (int q = 0; q < nQf; ++q)
             for (int i = 0; i < nB; ++i)
                 for (int j = 0; j < nB; ++j) E[i * nB + j] += desc.face_weights[q] * ps[q * nB + i] * pn[q * nB + j];
+        // (a function that vanishes on the face is tabulated as rounding noise there)
+        double big = 0.0;
+        for (int q = 0; q < nQf * nB; ++q) big = std::max(big, std::fabs(pn[q]));
+        for (int j = 0; j < nB; ++j) {
+            double most = 0.0;
+            for (int q = 0; q < nQf; ++q) most = std::max(most, std::fabs(pn[q * nB + j]));
+            op.pair_trace.push_back(most > 1e-13 * big);
+        }
         size_t off = op.pairs.size();
         op.pairs.resize(off + (size_t)nB * nB);
         matmul(nB, op.mass_inv.data(), E.data(), &op.pairs[off]);

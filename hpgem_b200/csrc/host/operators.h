@@ -38,6 +38,7 @@ struct HostOperators {
     std::vector<double> vol;        // [dim][nB][nB]
     std::vector<double> pairs;      // [n_pairs][nB][nB]
     int n_pairs = 0;
+    std::vector<uint8_t> pair_trace;  // [n_pairs][nB] whether the trial side's function does not vanish on the face
     std::vector<int32_t> nbr;       // [E][nfl]
     std::vector<int32_t> self_pair; // [E][nfl]
     std::vector<int32_t> nbr_pair;  // [E][nfl]
