@@ -27,7 +27,12 @@ SOURCES = sorted(glob.glob(os.path.join(CSRC, "*.cu"))) + [
 HEADERS = sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(glob.glob(os.path.join(CSRC, "host", "*.h"))) + [
     os.path.join(CSRC, "host", "simplex_rules.inc"),
     os.path.join(os.path.dirname(HERE), "include", "hpgem_b200.h")]
-FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--split-compile=0", "-Xcompiler", "-fPIC"]
+FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
+
+
+# sources of many template instances, whose optimiser runs on all cores (it compiles some
+# kernels of the other sources differently, measurably slower, so only these)
+SPLIT = ("stage_lane.cu", "batch_lane.cu")
 
 
 def nvcc():
@@ -64,7 +69,8 @@ def up_to_date():
 def _compile(src, verbose):
     o = _obj(src)
     tmp = o + ".tmp%d" % os.getpid()
-    cmd = [nvcc()] + FLAGS + (["-Xptxas=-v"] if verbose else []) + ["-c", src, "-o", tmp]
+    split = ["--split-compile=0"] if os.path.basename(src) in SPLIT else []
+    cmd = [nvcc()] + FLAGS + split + (["-Xptxas=-v"] if verbose else []) + ["-c", src, "-o", tmp]
     subprocess.run(cmd, check=True)
     os.replace(tmp, o)
     return o

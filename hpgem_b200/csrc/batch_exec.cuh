@@ -27,6 +27,8 @@
 #include <mutex>
 #include <tuple>
 
+#include "batch_items.cuh"
+
 namespace hgg {
 
 template <typename KT>
@@ -42,20 +44,6 @@ struct alignas(16) TensorItem {
     StageIOT<KT> io[2];
     TensorGeom geo;
     int64_t block0;
-    int slot;
-};
-template <typename KT>
-struct alignas(16) TensorLaneItem {
-    StageIOT<KT> io[2];
-    TensorLaneGeom g;
-    int64_t block0;  // first virtual block of kLaneWarps tiles
-    int slot;
-};
-template <typename KT>
-struct alignas(16) LaneItem {
-    StageIOT<KT> io[2];
-    LaneGeom g;
-    int64_t block0;  // first virtual block (= chunk)
     int slot;
 };
 template <typename KT>
@@ -82,35 +70,6 @@ struct alignas(16) LinearItem {
     int64_t block0;  // first virtual block (= tile)
     int slot;
 };
-
-// item whose virtual blocks contain vb: binary search of the items' first blocks,
-// which the class table keeps as one compact array after the block total (total[1 + m]
-// = item m's block0, ascending, total[1] = 0), so the probes stay in a few cache lines
-// instead of touching one item record each
-__device__ __forceinline__ int find_item(const int64_t *total, int n, int64_t vb) {
-    const int64_t *block0 = total + 1;
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (block0[mid] <= vb) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// The item of the virtual block in shared memory: the stage bodies read its fields
-// (pointers, coefficients, sizes) many times, which from shared memory costs what the
-// one-problem kernels pay for their parameters, not an L1 load each.  Ends with a
-// barrier; the caller's loop begins with one, so the previous block is done with it.
-template <typename Item>
-__device__ __forceinline__ const Item &item_to_shared(const Item *items, int i, Item &s_item) {
-    static_assert(sizeof(Item) % 16 == 0, "items are copied in 16-byte chunks");
-    const int4 *src = reinterpret_cast<const int4 *>(items + i);
-    int4 *dst = reinterpret_cast<int4 *>(&s_item);
-    for (int k = threadIdx.x; k < (int)(sizeof(Item) / 16); k += blockDim.x) dst[k] = src[k];
-    __syncthreads();
-    return s_item;
-}
 
 template <typename KT, int DIM, int NFL, int WAVE, int NB>
 __global__ void __launch_bounds__(256)
@@ -161,61 +120,6 @@ __global__ void __launch_bounds__(EPB *TensorConsts<P, DIM>::NB)
         __shared__ TensorItem<KT> s_it;
         const TensorItem<KT> &it = item_to_shared(items, i, s_it);
         tensor_stage_body<KT, P, DIM, EPB>(it.io[parity[slot]], it.geo, tc, vb - it.block0);
-    }
-}
-
-// one element per thread, a warp per tile, kLaneWarps tiles per virtual block
-constexpr int kLaneWarps = 4;
-template <typename KT, int P, int DIM, int NIN, bool FIN>
-__global__ void __launch_bounds__(32 * kLaneWarps)
-    grouped_tensor_lane(const TensorLaneItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
-                        const int *remaining) {
-    const int n = *n_items;
-    const int64_t nb = *total;
-    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
-        const int i = find_item(total, n, vb);
-        const int slot = items[i].slot;
-        __syncthreads();
-        if (remaining[slot] <= 0) continue;
-        __shared__ TensorLaneItem<KT> s_it;
-        const TensorLaneItem<KT> &it = item_to_shared(items, i, s_it);
-        const int64_t tile = (vb - it.block0) * kLaneWarps + (threadIdx.x >> 5);
-        if (tile < it.g.n_tiles) tensor_lane_body<KT, P, DIM, NIN, FIN>(it.io[parity[slot]], it.g, tile);
-    }
-}
-
-// simplices and the wave, one element per thread: a chunk of a member per virtual block
-template <typename KT, typename CT, typename ST, int DIM, int NFL, int NB>
-__global__ void __launch_bounds__(LaneShape<KT, CT, DIM, NFL, NB, true>::THREADS)
-    grouped_wave_lane(const LaneItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
-                      const int *remaining) {
-    const int n = *n_items;
-    const int64_t nb = *total;
-    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
-        const int i = find_item(total, n, vb);
-        const int slot = items[i].slot;
-        __syncthreads();
-        if (remaining[slot] <= 0) continue;
-        __shared__ LaneItem<KT> s_it;
-        const LaneItem<KT> &it = item_to_shared(items, i, s_it);
-        wave_lane_body<KT, CT, ST, DIM, NFL, NB>(it.io[parity[slot]], it.g, vb - it.block0);
-    }
-}
-
-template <typename KT, typename CT, int DIM, int NFL, int NB, int NIN>
-__global__ void __launch_bounds__(LaneShape<KT, CT, DIM, NFL, NB, false>::THREADS)
-    grouped_advection_lane(const LaneItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
-                           const int *remaining) {
-    const int n = *n_items;
-    const int64_t nb = *total;
-    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
-        const int i = find_item(total, n, vb);
-        const int slot = items[i].slot;
-        __syncthreads();
-        if (remaining[slot] <= 0) continue;
-        __shared__ LaneItem<KT> s_it;
-        const LaneItem<KT> &it = item_to_shared(items, i, s_it);
-        advection_lane_body<KT, CT, DIM, NFL, NB, NIN>(it.io[parity[slot]], it.g, vb - it.block0);
     }
 }
 
@@ -653,7 +557,6 @@ void class_kernel(const hgg_batch *b, Kern kern, unsigned grid, unsigned threads
     }
     kern<<<grid, threads, smem, s>>>(args...);
 }
-
 template <typename KT, int DIM, int NFL, int WAVE>
 void launch_grouped_dense(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
     const int nB = c.rep.nB;
@@ -712,65 +615,6 @@ int class_nin(const BatchClass &c, int st) {
     int n = 0;
     for (int j = 0; j < st; ++j) n += c.rk_a[st * c.S + j] != 0.0;
     return n;
-}
-
-template <typename KT>
-void launch_grouped_tensor_lane(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
-    tensor_lane_dispatch(c.dim, c.order, [&](auto p, auto d) {
-        lane_stage_shape(class_nin(c, st), st == c.S - 1, [&](auto nin, auto fin) {
-            class_kernel(b,
-                         grouped_tensor_lane<KT, decltype(p)::value, decltype(d)::value, decltype(nin)::value,
-                                             decltype(fin)::value>,
-                         grid, 32 * kLaneWarps, 0, s, static_cast<const TensorLaneItem<KT> *>(c.d_items[st]), c.d_n,
-                         c.d_total, b->d_parity, b->d_remaining);
-        });
-    });
-}
-
-template <typename KT, int DIM, int NFL, int WAVE>
-void launch_grouped_lane(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
-    dense_dispatch<DIM, NFL, WAVE>(c.rep.nB, [&](auto nbc) {
-        constexpr int NB = decltype(nbc)::value;
-        using CT = DenseCT<KT, NB>;
-        if constexpr (lane_size(DIM, NFL, WAVE, NB)) {
-            auto go = [&](auto kern, int threads, int smem) {
-                if (smem > 48 * 1024 - (int)sizeof(LaneItem<KT>))
-                    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-                class_kernel(b, kern, grid, threads, smem, s, static_cast<const LaneItem<KT> *>(c.d_items[st]), c.d_n,
-                             c.d_total, b->d_parity, b->d_remaining);
-            };
-            if constexpr (WAVE) {
-                using SH = LaneShape<KT, CT, DIM, NFL, NB, true>;
-                if (st > 0)
-                    go(grouped_wave_lane<KT, CT, CT, DIM, NFL, NB>, SH::THREADS,
-                       wave_lane_smem<KT, CT, CT, DIM, NFL, NB>(c.lane_bytes, SH::TILES));
-                else
-                    go(grouped_wave_lane<KT, CT, double, DIM, NFL, NB>, SH::THREADS,
-                       wave_lane_smem<KT, CT, double, DIM, NFL, NB>(c.lane_bytes, SH::TILES));
-            } else {
-                constexpr int threads = LaneShape<KT, CT, DIM, NFL, NB, false>::THREADS;
-                const int nin = class_nin(c, st);
-                if (nin == 0) go(grouped_advection_lane<KT, CT, DIM, NFL, NB, 0>, threads, c.lane_bytes);
-                else if (nin == 1) go(grouped_advection_lane<KT, CT, DIM, NFL, NB, 1>, threads, c.lane_bytes);
-                else go(grouped_advection_lane<KT, CT, DIM, NFL, NB, -1>, threads, c.lane_bytes);
-            }
-        }
-    });
-}
-
-template <typename KT>
-void launch_grouped_lane_any(const hgg_batch *b, const BatchClass &c, int st, unsigned grid, cudaStream_t s) {
-    const bool wave = c.physics != HGG_PHYSICS_ADVECTION;
-    switch (c.shape) {
-        case HGG_SHAPE_TRIANGLE:
-            wave ? launch_grouped_lane<KT, 2, 3, 1>(b, c, st, grid, s) : launch_grouped_lane<KT, 2, 3, 0>(b, c, st, grid, s);
-            break;
-        case HGG_SHAPE_TETRAHEDRON:
-            wave ? launch_grouped_lane<KT, 3, 4, 1>(b, c, st, grid, s) : launch_grouped_lane<KT, 3, 4, 0>(b, c, st, grid, s);
-            break;
-        case HGG_SHAPE_SQUARE: launch_grouped_lane<KT, 2, 4, 1>(b, c, st, grid, s); break;
-        case HGG_SHAPE_CUBE: launch_grouped_lane<KT, 3, 6, 1>(b, c, st, grid, s); break;
-    }
 }
 
 template <typename KT>
@@ -888,12 +732,11 @@ void launch_class_stage(hgg_batch *b, const BatchClass &c, int st, cudaStream_t 
                 c.mixed ? launch_grouped_wave<float, 3, 6>(b, c, st, grid, s) : launch_grouped_wave<double, 3, 6>(b, c, st, grid, s);
                 break;
         }
-    } else if (c.kind == KIND_LANE) {
-        if (c.mixed) launch_grouped_lane_any<float>(b, c, st, grid, s);
-        else launch_grouped_lane_any<double>(b, c, st, grid, s);
-    } else if (c.kind == KIND_TENSOR_LANE) {
-        if (c.mixed) launch_grouped_tensor_lane<float>(b, c, st, grid, s);
-        else launch_grouped_tensor_lane<double>(b, c, st, grid, s);
+    } else if (c.kind == KIND_LANE || c.kind == KIND_TENSOR_LANE) {
+        launch_class_lane(LaneClassStage{c.kind == KIND_TENSOR_LANE, c.mixed, c.dim, c.order, c.shape,
+                                         c.physics != HGG_PHYSICS_ADVECTION, c.rep.nB, st, class_nin(c, st),
+                                         st == c.S - 1, c.lane_bytes, c.d_items[st], c.d_n, c.d_total, b->d_parity,
+                                         b->d_remaining, grid, s, b->occ_query ? &b->occ_result : nullptr});
     } else if (c.kind == KIND_TENSOR) {
 #define HGG_GT(P)                                                  \
     case P:                                                        \

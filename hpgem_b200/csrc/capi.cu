@@ -66,11 +66,12 @@ int solution_to_host(hgg_handle *h, double *staging, double *out) {
 }
 
 void release_graphs(hgg_handle *h) {
-    for (auto &g : h->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    for (auto *graphs : {h->graph, h->graph_run})
+        for (int from = 0; from < 2; ++from)
+            if (graphs[from]) {
+                cudaGraphExecDestroy(graphs[from]);
+                graphs[from] = nullptr;
+            }
 }
 // ---- kernel dispatch ---------------------------------------------------------
 // The device vectors of a sum-factorised handle are already in tensor order
@@ -760,6 +761,32 @@ void destroy_handle(hgg_handle *h) {
 
 }  // namespace hgg
 
+namespace {
+// `steps` steps from sol[from] captured as one graph
+int capture_steps(hgg_handle *h, int from, int steps, double dt, cudaGraphExec_t *exec) {
+    cudaGraph_t g = nullptr;
+    HGG_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    const int64_t before = h->launches;
+    int rc = 0;
+    for (int s = 0; s < steps && !rc; ++s) rc = enqueue_step(h, (from + s) & 1, dt);
+    const cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
+    h->graph_launches = (h->launches - before) / steps;  // kernels of one captured step
+    h->launches = before;                                // capture does not launch
+    if (rc) {
+        if (g) cudaGraphDestroy(g);
+        return rc;
+    }
+    if (ce != cudaSuccess) return fail(h, HGG_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
+    const cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ie != cudaSuccess) {
+        *exec = nullptr;
+        return fail(h, HGG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
+    }
+    return 0;
+}
+}  // namespace
+
 extern "C" {
 
 int hgg_create(const hgg_problem_desc *desc, hgg_handle **out) {
@@ -837,38 +864,24 @@ int hgg_get_state(hgg_handle *h, int32_t vec, double *host) {
 int hgg_step(hgg_handle *h, double *time, double dt, int32_t nsteps) {
     if (!h || nsteps < 0) return fail(h, HGG_ERR_INVALID, "bad argument");
     if (nsteps == 0) return 0;
-    if (!(dt == h->graph_dt && h->store_last == h->graph_store_last && h->graph[0] && h->graph[1])) {
+    if (!(dt == h->graph_dt && h->store_last == h->graph_store_last)) {
         release_graphs(h);
-        for (int from = 0; from < 2; ++from) {
-            cudaGraph_t g = nullptr;
-            HGG_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-            int64_t before = h->launches;
-            int rc = enqueue_step(h, from, dt);
-            cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
-            h->graph_launches = h->launches - before;  // kernels of one captured step
-            h->launches = before;                      // capture does not launch
-            if (rc) {
-                if (g) cudaGraphDestroy(g);
-                return rc;
-            }
-            if (ce != cudaSuccess) return fail(h, HGG_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-            cudaError_t ie = cudaGraphInstantiate(&h->graph[from], g, 0);
-            cudaGraphDestroy(g);
-            if (ie != cudaSuccess) return fail(h, HGG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
-        }
         h->graph_dt = dt;
         h->graph_store_last = h->store_last;
     }
     if (h->src && !time) return fail(h, HGG_ERR_INVALID, "source terms need the time: pass a time");
-    for (int s = 0; s < nsteps; ++s) {
-        if (h->src) {  // the source values of this step's stage times
-            int rc = fill_sources(h, h->cur, *time, dt);
-            if (rc) return rc;
-        }
-        HGG_CUDA(h, cudaGraphLaunch(h->graph[h->cur], h->stream));
-        h->launches += h->graph_launches;
-        h->cur = 1 - h->cur;
-        if (time) *time += dt;
+    for (int s = 0; s < nsteps;) {
+        int rc;
+        if (h->src && (rc = fill_sources(h, h->cur, *time, dt))) return rc;  // of this step's stage times
+        // whole runs of steps while there are that many (a source is filled step by step)
+        const int run = !h->src && nsteps - s >= hgg_handle::kRunSteps ? hgg_handle::kRunSteps : 1;
+        cudaGraphExec_t *g = run > 1 ? &h->graph_run[h->cur] : &h->graph[h->cur];
+        if (!*g && (rc = capture_steps(h, h->cur, run, dt, g))) return rc;
+        HGG_CUDA(h, cudaGraphLaunch(*g, h->stream));
+        h->launches += run * h->graph_launches;
+        if (run % 2) h->cur = 1 - h->cur;
+        for (int i = 0; i < run && time; ++i) *time += dt;
+        s += run;
     }
     return 0;
 }

@@ -25,6 +25,13 @@ namespace hgg {
 
 constexpr int kMaxStages = 8;
 
+// Programmatic dependent launch (launch_chained): a stage's blocks may start while the
+// previous stage's last blocks still run.  chain_next lets the next stage's do so;
+// chain_wait returns when the previous stage has finished and its writes are visible, so
+// before it a kernel reads only what no stage writes (operators, geometry, indices).
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Linear combination inputs and the fused final update of one stage.
 // Inputs and outputs of one stage launch.  KT is the storage type of the
 // stage vectors: double in the FP64 form, float in the FP32-mixed form (the

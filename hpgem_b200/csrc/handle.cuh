@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/hpgem_b200.h"
@@ -114,8 +115,10 @@ struct hgg_handle {
     bool store_last = true;
     int64_t launches = 0;
     int64_t graph_launches = 0;  // kernels in one captured step
-    // graph of one full step, per starting buffer, valid for (dt, store_last)
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    // graphs of one step and of kRunSteps steps, per starting buffer, valid for (dt,
+    // store_last); made when first needed
+    static constexpr int kRunSteps = 8;
+    cudaGraphExec_t graph[2] = {nullptr, nullptr}, graph_run[2] = {nullptr, nullptr};
     double graph_dt = 0.0;
     bool graph_store_last = true;
     std::string err = "no error";
@@ -164,6 +167,28 @@ void release_graphs(hgg_handle *h);
 // the current solution in hpGEM order with no kernel on the device: one copy of the
 // device vector into `staging` (pinned, h->N_alloc doubles), the layout change on the host
 int solution_to_host(hgg_handle *h, double *staging, double *out);
+
+// Launch of a stage kernel that calls chain_next and chain_wait: its start overlaps the
+// previous kernel's end on the same stream (anything else before it is waited for in
+// full), which takes most of the gap between two stages out.  Per RK4 step: 32^2
+// quadrilaterals at p = 2 12.7 -> 9.1 us, triangles 192 x 160 at p = 3 22.6 -> 17.9, the
+// FP32 wave on 14 x 18 x 12 x 5 tetrahedra at p = 3 160 -> 154.  (Letting the next stage
+// start at a kernel's beginning instead of before its outputs spreads its blocks unevenly
+// over the SMs: the triangles took 23.7.)
+template <typename... K, typename... A>
+void launch_chained(void (*kern)(K...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);  // (the caller checks cudaGetLastError)
+}
 
 template <int P, int DIM>
 TensorConsts<P, DIM> tensor_consts(const HostOperators &op) {

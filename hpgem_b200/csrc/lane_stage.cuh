@@ -109,6 +109,7 @@ __device__ __forceinline__ void column_load(const CT *a, CT (&o)[RB]) {
 template <typename KT, typename CT, int F, int RB>
 __device__ __forceinline__ void lane_output(const StageIOT<KT> &io, int64_t idx, int64_t step, int rows,
                                             const CT (&k)[F][RB]) {
+    chain_next();
     if (io.kout) {
         KT *out = io.kout + idx;
 #pragma unroll
@@ -217,6 +218,7 @@ __device__ __forceinline__ void wave_lane_body(const StageIOT<KT> &io, const Lan
     for (int f = 0; f < NFL; ++f) nb[f] = __ldg(g.nbr + (tile * NFL + f) * 32 + lane);
 
     for (int i = threadIdx.x; i < g.group_bytes / 16; i += blockDim.x) cp_async<16>(lane_shared + 16 * i, table + 16 * i);
+    chain_wait();
     if (active)
         for (int i = rw * 32 + lane; i < (int)sizeof(ST) * 2 * R; i += 32 * RW)
             cp_async<16>(reinterpret_cast<unsigned char *>(own) + 16 * i,
@@ -533,6 +535,7 @@ __device__ __forceinline__ void advection_lane_body(const StageIOT<KT> &io, cons
     int32_t nb[NFL];
 #pragma unroll
     for (int f = 0; f < NFL; ++f) nb[f] = __ldg(g.nbr + (tile * NFL + f) * 32 + lane);
+    chain_wait();
     auto neighbour = [&](int f) {  // first coefficient of the neighbour across face f (any f of the block)
         int32_t n = nb[0];
 #pragma unroll

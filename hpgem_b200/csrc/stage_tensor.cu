@@ -45,8 +45,9 @@ int launch_tensor_lane(hgg_handle *h, const StageIOT<KT> &io) {
     const unsigned blocks = (unsigned)((g.n_tiles + warps - 1) / warps);
     const bool ok = tensor_lane_dispatch(h->op.dim, h->op.order, [&](auto p, auto d) {
         lane_stage_shape(io.nin, io.unew != nullptr, [&](auto nin, auto fin) {
-            tensor_lane<KT, decltype(p)::value, decltype(d)::value, decltype(nin)::value, decltype(fin)::value>
-                <<<blocks, 32 * warps, 0, h->stream>>>(io, g);
+            launch_chained(
+                tensor_lane<KT, decltype(p)::value, decltype(d)::value, decltype(nin)::value, decltype(fin)::value>, blocks,
+                32 * warps, 0, h->stream, io, g);
         });
     });
     return ok ? 0 : fail(h, HGG_ERR_UNSUPPORTED, "lane kernel: order out of range");

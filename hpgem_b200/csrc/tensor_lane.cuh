@@ -48,6 +48,7 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
 #pragma unroll
     for (int c = 0; c < DIM; ++c) nb[c] = g.side[c] >= 0 ? __ldg(g.nbr + (tile * DIM + c) * 32 + lane) : 0;
 
+    chain_wait();
     // stage input of N coefficients at base + 32 pos(i), formed in FP64 and rounded once;
     // every vector's loads are issued together
     auto input = [&](auto count, auto pos, int64_t from, CT *out) {
@@ -91,6 +92,7 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
               },
               from, tr[c]);
     }
+    chain_next();
     double fu[FIN ? NB : 1];
     if (FIN) {
 #pragma unroll
