@@ -380,11 +380,12 @@ void lane_setup(hgg_handle *h, LaneMesh &m, LaneTables &t) {
     const HostOperators &op = h->op;
     const bool wave = op.physics != HGG_PHYSICS_ADVECTION;
     if (!lane_size(op.dim, op.nfl, wave, op.nB) || op.nB != lane_basis(op.dim, op.nfl, op.order)) return;
-    // 64-bit handles take the folded tables; the FP32 form keeps its order of operations, and
-    // its folded triangles (p = 5) the stored-matrix tiles
+    // 64-bit handles take the folded tables; the FP32 form keeps its order of operations
     const bool folded = !h->mixed;
     const int elem_bytes = folded || op.nB > kMixedFp32MaxBasis ? 8 : 4;
-    if (h->mixed && !wave && op.shape == HGG_SHAPE_TRIANGLE && op.nB >= 21) return;
+    // (the FP32 form above kMixedFp32MaxBasis functions contracts in 64 bits with plain
+    // tables: tetrahedra at p = 4 on 6^3 x 5 took 118 us per step against the row kernel's 51)
+    if (h->mixed && !wave && op.nB > kMixedFp32MaxBasis) return;
     // a block takes several tiles of a group once every SM has two such blocks: the group's
     // table is then read from L2 once for all of them
     const int most = std::max(1, 4 / lane_warps(op.nB, wave ? lane_wave_rows(folded) : kLaneAdvRows));

@@ -126,7 +126,7 @@ bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int co
         dst[n] = (uint64_t)(int64_t)e;
         return true;
     };
-    const size_t most = (size_t)op.nE / 16 + 64;  // more groups than this cannot fill tiles
+    const size_t most = (size_t)op.nE / 10 + 296;  // more groups than this take too much padding
     for (int64_t e = 0; e < op.nE; ++e) {
         uint64_t *k = key.data();
         for (int f = 0; f < nf; ++f) {
@@ -155,9 +155,10 @@ bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int co
     int64_t tiles = 0;
     for (int64_t c : count) tiles += (c + 31) / 32;
     const int64_t pad = tiles * 32 - op.nE;
-    // padded slots cost idle lanes and memory in every vector: at most half as many as
-    // elements (or two tiles), and within spare_bytes per element and 4 MB
-    if (pad > std::max<int64_t>(op.nE / 2, 64)) return false;
+    // padded slots cost idle lanes and memory in every vector: at most twice as many as
+    // elements (a full tile's element costs a third of the general kernels') unless all
+    // tiles run at once, and within spare_bytes per element and 4 MB
+    if (pad > 2 * op.nE && tiles > 2 * 148) return false;
     if ((double)pad * R * coefficient_bytes > (double)spare_bytes * (double)op.nE + 4e6) return false;
     if (tiles > INT32_MAX / 32) return false;
     m.n_slots = tiles * 32;

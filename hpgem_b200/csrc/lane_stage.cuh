@@ -77,13 +77,20 @@ struct LaneShape {
     static constexpr int THREADS = 32 * RW * TILES;
 };
 
-// the group's table into shared memory (every thread of the block); ends with a barrier
-__device__ __forceinline__ void lane_stage_table(const LaneGeom &g, int group, unsigned char *dst) {
-    const int4 *src = reinterpret_cast<const int4 *>(g.tables + (size_t)group * g.group_bytes);
-    int4 *d = reinterpret_cast<int4 *>(dst);
-#pragma unroll 4
-    for (int i = threadIdx.x; i < g.group_bytes / 16; i += blockDim.x) d[i] = __ldg(src + i);
-    __syncthreads();
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+// the group's table into shared memory, by every thread of the block (not committed)
+__device__ __forceinline__ void request_table(const LaneGeom &g, const unsigned char *table, unsigned char *dst) {
+    for (int i = threadIdx.x; i < g.group_bytes / 16; i += blockDim.x) cp_async<16>(dst + 16 * i, table + 16 * i);
 }
 
 // acc[i] += a[i] x, a: RB entries of an operator column in shared memory (a broadcast)
@@ -171,18 +178,6 @@ __device__ __forceinline__ double lane_add(double a, double b) { return __dadd_r
 __device__ __forceinline__ float lane_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double lane_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void *dst, const void *src) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
-}
-
 // dynamic shared memory: the group's table, then per tile the elements' input [R][32] and
 // the ring of faces [V][NC][32], in elements of the source type; NC columns of a neighbour:
 // its trace functions in a folded table, any with a nonzero entry in a plain one
@@ -217,7 +212,7 @@ __device__ __forceinline__ void wave_lane_body(const StageIOT<KT> &io, const Lan
 #pragma unroll
     for (int f = 0; f < NFL; ++f) nb[f] = __ldg(g.nbr + (tile * NFL + f) * 32 + lane);
 
-    for (int i = threadIdx.x; i < g.group_bytes / 16; i += blockDim.x) cp_async<16>(lane_shared + 16 * i, table + 16 * i);
+    request_table(g, table, lane_shared);
     chain_wait();
     if (active)
         for (int i = rw * 32 + lane; i < (int)sizeof(ST) * 2 * R; i += 32 * RW)
@@ -518,25 +513,47 @@ int wave_lane_smem(int group_bytes, int tiles) {
 // ---- advection ----------------------------------------------------------------------
 // NIN: stage vectors in the stage input (0, 1, or -1 for a count read from io); they are
 // combined on loading, in FP64 and rounded once, so no vector is formed ahead.
+// Small elements (REG) hold all their inputs in registers: one round of loads, in flight
+// with the table, then arithmetic alone.  Larger ones load up to ten columns at a time.
 template <typename KT, typename CT, int DIM, int NFL, int NB, int NIN>
 __device__ __forceinline__ void advection_lane_body(const StageIOT<KT> &io, const LaneGeom &g, int64_t block) {
     using SH = LaneShape<KT, CT, DIM, NFL, NB, false>;
     constexpr int RW = SH::RW, RB = SH::RB, RBP = SH::RBP, NFC = SH::NFC;
-    constexpr int CH = 5;  // columns loaded together
+    constexpr int NC = SH::FOLDED ? NFC : NB;  // columns of a face
+    constexpr bool REG = NB <= (SH::FOLDED ? 21 : 15);
+    constexpr bool FACES_AHEAD = REG && NFL * NC <= 40;
+    constexpr int CH = REG ? (NB > NC ? NB : NC) : 10;  // columns loaded together
+    constexpr int OPS = (SH::FOLDED ? NB + NFL * NFC : (DIM + NFL) * NB) * RBP;  // of one row warp
     extern __shared__ __align__(16) unsigned char lane_shared[];
     const LaneChunk ch = g.chunks[block];
-    lane_stage_table(g, ch.group, lane_shared);
+    const unsigned char *table = g.tables + (size_t)ch.group * g.group_bytes;
+    request_table(g, table, lane_shared);
+    cp_async_commit();
+    // folded: number of inflow faces, [NFL] face, [NFL][NFC] column; plain: [NFL] upwind mode
+    // (read from global memory: the table is in flight)
+    const int32_t *head = reinterpret_cast<const int32_t *>(table + sizeof(CT) * RW * OPS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int local = warp / RW, rw = warp % RW;
-    if (local >= ch.tiles) return;
-    const int64_t tile = ch.tile0 + local;
+    const bool active = local < ch.tiles;
+    const int64_t tile = ch.tile0 + (active ? local : 0);
     const int64_t base = tile * (32 * NB) + lane;
-    const int rows = min(RB, NB - rw * RB);
     int32_t nb[NFL];
 #pragma unroll
     for (int f = 0; f < NFL; ++f) nb[f] = __ldg(g.nbr + (tile * NFL + f) * 32 + lane);
-    chain_wait();
-    auto neighbour = [&](int f) {  // first coefficient of the neighbour across face f (any f of the block)
+    const double *geo = g.geo + tile * (32 * (DIM + NFL)) + lane;  // plain
+    CT ahat[DIM], sigma[NFL];
+    if constexpr (!SH::FOLDED) {
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) ahat[c] = (CT)ldg_f64(geo + 32 * c);
+#pragma unroll
+        for (int f = 0; f < NFL; ++f) sigma[f] = (CT)ldg_f64(geo + 32 * (DIM + f));
+    }
+    // the k-th neighbour that enters the stage: the face, or -1
+    auto inflow = [&](int k) {
+        if constexpr (SH::FOLDED) return k < __ldg(head) ? __ldg(head + 1 + k) : -1;
+        else return __ldg(head + k) == 2 ? k : -1;
+    };
+    auto neighbour = [&](int f) {  // first coefficient of the neighbour across face f
         int32_t n = nb[0];
 #pragma unroll
         for (int k = 1; k < NFL; ++k) n = f == k ? nb[k] : n;
@@ -547,7 +564,7 @@ __device__ __forceinline__ void advection_lane_body(const StageIOT<KT> &io, cons
         return (int64_t)(n >> 5) * (32 * NB) + (n & 31);
     };
     // stage input of up to CH coefficients at from + offset(i), i < count
-    auto input = [&](int64_t from, int count, auto offset, CT (&x)[CH]) {
+    auto input = [&](int64_t from, int count, auto offset, CT *x) {
         double v[CH];
 #pragma unroll
         for (int i = 0; i < CH; ++i) v[i] = i < count ? ldg_f64(io.u + from + offset(i)) : 0.0;
@@ -565,105 +582,120 @@ __device__ __forceinline__ void advection_lane_body(const StageIOT<KT> &io, cons
 #pragma unroll
         for (int i = 0; i < CH; ++i) x[i] = (CT)v[i];
     };
-    const CT *ops = reinterpret_cast<const CT *>(lane_shared);
+    auto own_input = [&](int j, CT *x) { input(base, min(NB - j, CH), [=](int i) { return 32 * (j + i); }, x); };
+    auto face_input = [&](int k, int f, int j, CT *x) {
+        const int64_t from = neighbour(f);
+        if constexpr (SH::FOLDED) {
+            const int32_t *cols = head + 1 + NFL + k * NFC + j;
+            input(from, min(NC - j, CH), [=](int i) { return __ldg(cols + i); }, x);
+        } else {
+            input(from, min(NC - j, CH), [=](int i) { return 32 * (j + i); }, x);
+        }
+    };
+    chain_wait();
+    CT xo[CH], xn[FACES_AHEAD ? NFL : 1][CH];
+    if (active) {
+        own_input(0, xo);
+        if constexpr (FACES_AHEAD) {
+#pragma unroll
+            for (int k = 0; k < NFL; ++k) {
+                const int f = inflow(k);
+                if (f >= 0) face_input(k, f, 0, xn[k]);
+            }
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // the table
+    if (!active) return;
+    const int rows = min(RB, NB - rw * RB);
+    const CT *op = reinterpret_cast<const CT *>(lane_shared) + rw * OPS;
     CT acc[1][RB];
 #pragma unroll
     for (int i = 0; i < RB; ++i) acc[0][i] = CT(0);
+    // out += the operator's columns j .. j + CH (of n) times x; stride: entries between columns
+    auto columns = [&](const CT *a, int stride, int n, const CT *x, CT *out) {
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+            if (q >= n) continue;
+            CT o[RB];
+            column_load<RB>(a + q * stride, o);
+#pragma unroll
+            for (int i = 0; i < RB; ++i) out[i] += o[i] * x[q];
+        }
+    };
     if constexpr (SH::FOLDED) {
-        constexpr int OPS = (NB + NFL * NFC) * RBP;
-        const double *op = ops + rw * OPS;
-        const int32_t *head = reinterpret_cast<const int32_t *>(ops + RW * OPS);  // faces, [NFL] face, [NFL][NFC] column
-        auto columns = [&](const double *a, int count, const CT (&x)[CH]) {
-#pragma unroll
-            for (int q = 0; q < CH; ++q) {
-                if (q >= count) continue;
-                double o[RB];
-                column_load<RB>(a + q * RBP, o);
-#pragma unroll
-                for (int i = 0; i < RB; ++i) acc[0][i] += o[i] * x[q];
+        columns(op, RBP, NB, xo, acc[0]);
+        if constexpr (!REG) {
+#pragma unroll 1
+            for (int j = CH; j < NB; j += CH) {
+                own_input(j, xo);
+                columns(op + j * RBP, RBP, NB - j, xo, acc[0]);
             }
-        };
-#pragma unroll 2
-        for (int j = 0; j < NB; j += CH) {
-            double x[CH];
-            input(base, NB - j, [=](int i) { return 32 * (j + i); }, x);
-            columns(op + j * RBP, NB - j, x);
         }
         op += NB * RBP;
-        const int faces = head[0];
+        if constexpr (FACES_AHEAD) {
+#pragma unroll
+            for (int k = 0; k < NFL; ++k)
+                if (inflow(k) >= 0) columns(op + k * NC * RBP, RBP, NC, xn[k], acc[0]);
+        } else {
 #pragma unroll 1
-        for (int k = 0; k < faces; ++k, op += NFC * RBP) {
-            const int64_t from = neighbour(head[1 + k]);
-            const int32_t *cols = head + 1 + NFL + k * NFC;
-#pragma unroll 2
-            for (int j = 0; j < NFC; j += CH) {
-                double x[CH];
-                input(from, NFC - j, [=](int i) { return cols[j + i]; }, x);
-                columns(op + j * RBP, NFC - j, x);
+            for (int k = 0; k < NFL; ++k) {
+                const int f = inflow(k);
+                if (f < 0) break;
+#pragma unroll 1
+                for (int j = 0; j < NC; j += CH) {
+                    face_input(k, f, j, xo);
+                    columns(op + (k * NC + j) * RBP, RBP, NC - j, xo, acc[0]);
+                }
             }
         }
     } else {
         // the row kernel's order of operations: the axes' sums, then the faces' one after the other
-        constexpr int OPS = (DIM + NFL) * NB * RBP;
-        const CT *op = ops + rw * OPS;
-        const int32_t *mode = reinterpret_cast<const int32_t *>(ops + RW * OPS);
-        const double *geo = g.geo + tile * (32 * (DIM + NFL)) + lane;
-        {
-            CT s[DIM][RB];
+        CT s[DIM][RB];
 #pragma unroll
-            for (int c = 0; c < DIM; ++c)
+        for (int c = 0; c < DIM; ++c) {
 #pragma unroll
-                for (int i = 0; i < RB; ++i) s[c][i] = CT(0);
-#pragma unroll 1
-            for (int j = 0; j < NB; j += CH) {
-                CT x[CH];
-                input(base, NB - j, [=](int i) { return 32 * (j + i); }, x);
-#pragma unroll
-                for (int q = 0; q < CH; ++q) {
-                    if (j + q >= NB) continue;
-#pragma unroll
-                    for (int c = 0; c < DIM; ++c) {
-                        CT o[RB];
-                        column_load<RB>(op + ((j + q) * DIM + c) * RBP, o);
-#pragma unroll
-                        for (int i = 0; i < RB; ++i) s[c][i] += o[i] * x[q];
-                    }
-                }
-            }
-            CT ahat[DIM];
-#pragma unroll
-            for (int c = 0; c < DIM; ++c) ahat[c] = (CT)ldg_f64(geo + 32 * c);
-#pragma unroll
-            for (int c = 0; c < DIM; ++c)
-#pragma unroll
-                for (int i = 0; i < RB; ++i) acc[0][i] += ahat[c] * s[c][i];
+            for (int i = 0; i < RB; ++i) s[c][i] = CT(0);
+            columns(op + c * RBP, DIM * RBP, NB, xo, s[c]);
         }
+        if constexpr (!REG) {
+#pragma unroll 1
+            for (int j = CH; j < NB; j += CH) {
+                own_input(j, xo);
+#pragma unroll
+                for (int c = 0; c < DIM; ++c) columns(op + (j * DIM + c) * RBP, DIM * RBP, NB - j, xo, s[c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < DIM; ++c)
+#pragma unroll
+            for (int i = 0; i < RB; ++i) acc[0][i] += ahat[c] * s[c][i];
         op += DIM * NB * RBP;
-#pragma unroll 1
-        for (int f = 0; f < NFL; ++f, op += NB * RBP) {
-            const int md = mode[f];
+        auto flux = [&](int f, const CT *t) {  // each face's rounded, then added
+#pragma unroll
+            for (int i = 0; i < RB; ++i) acc[0][i] = lane_add(acc[0][i], -lane_mul(sigma[f], t[i]));
+        };
+#pragma unroll
+        for (int f = 0; f < NFL; ++f) {
+            const int md = __ldg(head + f);
             if (md != 1 && md != 2) continue;
-            const int64_t from = md == 1 ? base : neighbour(f);
-            CT s[RB];
+            CT t[RB];
 #pragma unroll
-            for (int i = 0; i < RB; ++i) s[i] = CT(0);
+            for (int i = 0; i < RB; ++i) t[i] = CT(0);
+            const CT *a = op + f * NB * RBP;
+            if constexpr (FACES_AHEAD) {
+                if (md == 1) columns(a, RBP, NB, xo, t);
+                else columns(a, RBP, NB, xn[f], t);
+            } else {
 #pragma unroll 1
-            for (int j = 0; j < NB; j += CH) {
-                CT x[CH];
-                input(from, NB - j, [=](int i) { return 32 * (j + i); }, x);
-#pragma unroll
-                for (int q = 0; q < CH; ++q) {
-                    if (j + q >= NB) continue;
-                    CT o[RB];
-                    column_load<RB>(op + (j + q) * RBP, o);
-#pragma unroll
-                    for (int i = 0; i < RB; ++i) s[i] += o[i] * x[q];
+                for (int j = 0; j < NB; j += CH) {
+                    CT x[CH];
+                    if (md == 1) own_input(j, x);
+                    else face_input(f, f, j, x);
+                    columns(a + j * RBP, RBP, NB - j, x, t);
                 }
             }
-            const CT sg = (CT)ldg_f64(geo + 32 * (DIM + f));
-#pragma unroll
-            for (int i = 0; i < RB; ++i)
-                acc[0][i] = lane_add(acc[0][i], -lane_mul(sg, s[i]));
+            flux(f, t);
         }
     }
     lane_output<KT, CT, 1, RB>(io, base + 32 * (rw * RB), 0, rows, acc);

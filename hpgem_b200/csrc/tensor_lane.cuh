@@ -104,6 +104,23 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
             for (int i = 0; i < NB; ++i) fu[i] += bj * ldg_k(kj + 32 * i);
         }
     }
+    // FP32 form: the rounded fluxes of every face
+    CT flux[DIM][2][std::is_same_v<CT, float> ? NF : 1];
+    if constexpr (std::is_same_v<CT, float>) {
+#pragma unroll
+        for (int c = 0; c < DIM; ++c)
+#pragma unroll
+            for (int sd = 0; sd < 2; ++sd) {
+                const int stride = c == 0 ? 1 : (c == 1 ? NP : NP * NP);
+                const bool in = g.side[c] == sd, out = (g.outflow[c] >> sd) & 1;
+#pragma unroll
+                for (int m = 0; m < NF; ++m) {
+                    const int lo = m % NP, hi = m / NP;
+                    const int pos = c == 0 ? NP * lo + NP * NP * hi : (c == 1 ? lo + NP * NP * hi : lo + NP * hi);
+                    flux[c][sd][m] = in ? g.sigma[c][sd] * tr[c][m] : (out ? g.sigma[c][sd] * w[pos + sd * stride] : CT(0));
+                }
+            }
+    }
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
         const int a[3] = {i % NP, (i / NP) % NP, DIM == 3 ? i / (NP * NP) : 0};
@@ -126,14 +143,9 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
             // the general kernel's order: the faces one after the other, each flux rounded
 #pragma unroll
             for (int c = 0; c < DIM; ++c) {
-                const int stride = c == 0 ? 1 : (c == 1 ? NP : NP * NP);
                 const int m = c == 0 ? a[1] + NP * a[2] : (c == 1 ? a[0] + NP * a[2] : a[0] + NP * a[1]);
 #pragma unroll
-                for (int sd = 0; sd < 2; ++sd) {
-                    const CT own = g.sigma[c][sd] * w[i + (sd - a[c]) * stride];
-                    const CT flux = g.side[c] == sd ? g.sigma[c][sd] * tr[c][m] : ((g.outflow[c] >> sd) & 1 ? own : CT(0));
-                    r -= g.lift[sd][a[c]] * flux;
-                }
+                for (int sd = 0; sd < 2; ++sd) r -= g.lift[sd][a[c]] * flux[c][sd][m];
             }
         }
         if (io.kout) io.kout[base + 32 * i] = r;

@@ -78,11 +78,11 @@ def test_variant_change_keeps_every_vector(precision):
 # Simplices and the wave: (cells, triangular, order, physics).  Meshes whose groups fill
 # whole tiles, leave the last tile partly filled, and (sides 2 mod 4) have odd groups along
 # the periodic wrap; every basis size of the two kernels.
-WAVES = [([24, 24], True, p) for p in (1, 2, 3, 4, 5)] + [([26, 22], True, 2), ([6, 6], False, 1),
+WAVES = [([24, 24], True, p) for p in (1, 2, 3, 4, 5)] + [([26, 22], True, 2), ([6, 6], False, 1), ([4, 4], True, 2), ([2, 2, 2], True, 2), ([4, 4, 4], True, 4),
          ([9, 7], False, 2), ([12, 11], False, 3), ([8, 9], False, 4), ([7, 8], False, 5),
          ([8, 8, 8], True, 1), ([8, 8, 8], True, 2), ([14, 10, 12], True, 2), ([8, 8, 8], True, 3),
          ([8, 8, 8], True, 4), ([5, 4, 3], False, 1), ([4, 3, 5], False, 2)]
-ADVECTIONS = [([24, 24], True, p) for p in (1, 2, 3, 4, 5)] + [([34, 30], True, 3)] + \
+ADVECTIONS = [([24, 24], True, p) for p in (1, 2, 3, 4, 5)] + [([34, 30], True, 3), ([6, 4], True, 3), ([10, 10], True, 5), ([4, 4, 4], True, 2)] + \
              [([8, 8, 8], True, p) for p in (1, 2, 3, 4, 5)]
 
 
