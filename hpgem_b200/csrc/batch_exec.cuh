@@ -157,6 +157,24 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// the pipelined form (a stage input of one vector): two blocks per tile
+template <typename KT, bool WIDE, bool PAIRS>
+__global__ void __launch_bounds__(kLinPipeThreads, lin_pipe_blocks(WIDE))
+    grouped_linear_pipe(const LinearItem<KT> *items, const int *n_items, const int64_t *total, const int *parity,
+                        const int *remaining) {
+    const int n = *n_items;
+    const int64_t nb = 2 * *total;
+    for (int64_t vb = blockIdx.x; vb < nb; vb += gridDim.x) {
+        const int i = find_item(total, n, vb >> 1);
+        const int slot = items[i].slot;
+        __syncthreads();
+        if (remaining[slot] <= 0) continue;
+        __shared__ LinearItem<KT> s_it;
+        const LinearItem<KT> &it = item_to_shared(items, i, s_it);
+        linear_pipe_body<KT, WIDE, PAIRS>(it.io[parity[slot]], it.g, it.t, vb - 2 * it.block0);
+    }
+}
+
 // the tiles of all members of a class, for the persistent tensor-core kernel
 struct UmmaGroupedTiles {
     const UmmaItem *items;
@@ -235,6 +253,7 @@ struct BatchClass {
     std::vector<double> rk_a, rk_b;
     // members and launch shape
     std::vector<int> slots;
+    bool chain = false;   // stored-matrix tiles: each stage forms the next one's input
     int lane_bytes = 0;   // lane kernels of simplices and the wave: bytes of a group's table
     int epb = 1;          // dense: elements per block
     int ctas_per_sm = 2;  // persistent CTAs per SM
@@ -342,7 +361,7 @@ bool same_class(const BatchClass &c, const hgg_handle *h) {
     return c.kind == batch_kind(h) && c.shape == h->op.shape && c.order == h->op.order && c.dim == h->op.dim &&
            c.physics == h->op.physics && c.mixed == h->mixed && c.S == h->S && c.rk_a == h->rk_a &&
            c.rk_b == h->rk_b &&
-           (c.kind != KIND_LANE || c.rep.nB == h->op.nB) &&
+           (c.kind != KIND_LANE || c.rep.nB == h->op.nB) && (c.kind != KIND_LINEAR || c.rows == h->lin_R) &&
            (c.kind != KIND_UMMA || (c.precision == h->precision && c.rows == h->lin_R && c.lslots == h->lin_slots));
 }
 
@@ -393,7 +412,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     if (c.kind == KIND_DENSE || c.kind == KIND_WAVE_TILES) {
         DenseItem<KT> it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.g = dense_geom(h, c.epb);
         it.tiles = c.kind == KIND_WAVE_TILES ? h->d_group_tiles : nullptr;
         it.block0 = block0;
@@ -402,7 +421,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     } else if (c.kind == KIND_UMMA) {
         UmmaItem it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<float>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<float>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.a = UmmaArgs{h->d_umma_img, h->d_umma_planes, h->d_umma_tile_elems, h->d_umma_tile_mats, h->d_lin_nbr,
                         h->umma_tiles, h->lin_mats, kUmmaPolls};
         it.block0 = block0;
@@ -411,7 +430,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     } else if (c.kind == KIND_LINEAR) {
         LinearItem<KT> it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.g = LinearGeom{h->d_lin_table, h->d_lin_table_rm, h->d_lin_table_f, h->d_lin_self, h->d_lin_nbr,
                           h->d_lin_mat, h->lin_R, h->lin_slots, std::max(1, 256 / h->lin_R), h->lin_mats};
         it.t = LinearTiles{h->d_lin_tile_elems, h->d_lin_tile_mats};
@@ -421,7 +440,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     } else if (c.kind == KIND_LANE) {
         LaneItem<KT> it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.g = h->lgeo;
         it.block0 = block0;
         it.slot = slot;
@@ -429,7 +448,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     } else if (c.kind == KIND_TENSOR_LANE) {
         TensorLaneItem<KT> it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.g = h->tlane;
         it.block0 = block0;
         it.slot = slot;
@@ -437,7 +456,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     } else if (c.kind == KIND_TENSOR) {
         TensorItem<KT> it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.geo = TensorGeom{h->d_ahat, h->d_tnbr, h->d_tmode, h->d_tsigma};
         it.block0 = block0;
         it.slot = slot;
@@ -445,7 +464,7 @@ void fill_member(const hgg_batch *b, const BatchClass &c, int slot, int stage, i
     } else {
         SliceItem<KT> it{};
         for (int par = 0; par < 2; ++par)
-            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status);
+            it.io[par] = make_stage_io<KT>(h, par ? 1 - base : base, b->dt[slot], stage, b->d_status, true);
         it.geo = h->d_slice_geo;
         it.block0 = block0;
         it.slot = slot;
@@ -706,6 +725,20 @@ void launch_class_stage(hgg_batch *b, const BatchClass &c, int st, cudaStream_t 
             tiles(KB16{});
         }
         if (!b->occ_query) b->launches++;  // the planes launch
+    } else if (c.kind == KIND_LINEAR && (st == 0 || c.chain)) {
+        auto go = [&](auto kt) {
+            using KT = decltype(kt);
+            lin_pipe_dispatch(c.rows, nullptr, [&](auto wide, auto pairs) {
+                constexpr bool W = decltype(wide)::value, P = decltype(pairs)::value;
+                cudaFuncSetAttribute(grouped_linear_pipe<KT, W, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     lin_pipe_smem(W));
+                class_kernel(b, grouped_linear_pipe<KT, W, P>, 2 * grid, kLinPipeThreads, lin_pipe_smem(W), s,
+                             static_cast<const LinearItem<KT> *>(c.d_items[st]), c.d_n, c.d_total, b->d_parity,
+                             b->d_remaining);
+            });
+        };
+        if (c.mixed) go(float{});
+        else go(double{});
     } else if (c.kind == KIND_LINEAR) {
         if (c.mixed)
             class_kernel(b, grouped_linear<float>, grid, 256, 0, s, static_cast<const LinearItem<float> *>(c.d_items[st]),
@@ -1097,6 +1130,7 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
         c.rows = h->lin_R;
         c.lslots = h->lin_slots;
         c.lane_bytes = h->lgeo.group_bytes;
+        c.chain = lin_forms_input(h, true);
         c.rep.shape = h->op.shape;
         c.rep.dim = h->op.dim;
         c.rep.order = h->op.order;

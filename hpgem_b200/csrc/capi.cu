@@ -220,12 +220,7 @@ bool group_wave_wanted(const hgg_handle *h) {
 }
 
 bool forms_next_input(const hgg_handle *h) {
-    if (h->lane || !h->d_win[0] || h->src || !group_wave_wanted(h)) return false;
-    const int S = h->S;
-    for (int i = 1; i < S; ++i)
-        for (int j = 0; j < i; ++j)
-            if ((h->rk_a[i * S + j] != 0.0) != (j == i - 1)) return false;
-    return true;
+    return !h->lane && h->d_win[0] && !h->src && group_wave_wanted(h) && chain_tableau(h);
 }
 
 template <typename KT>
@@ -709,6 +704,9 @@ int attach_linear(hgg_handle *h, const LinearSystem &sys, int tiles_only) {
             (rc = upload(h, tmat, &h->d_lin_tile_mats)))
             return rc;
         h->lin_tiles = n_tiles;
+        if (u_tiles == 0)
+            for (int i = 0; i < 2; ++i)
+                if ((rc = alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_lin_win[i]))) return rc;
     }
     if (u_tiles > 0) {
         // operand images of every distinct matrix: hi part then lo part, each NP x KP in the

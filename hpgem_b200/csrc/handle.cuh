@@ -92,6 +92,7 @@ struct hgg_handle {
     double *d_lin_table_rm = nullptr;
     int32_t *d_lin_tile_elems = nullptr, *d_lin_tile_mats = nullptr;
     int64_t lin_tiles = 0;
+    double *d_lin_win[2] = {nullptr, nullptr};  // stage inputs formed ahead (tiles, see lin_forms_input)
     int lin_min_rows = hgg::kLinTileMinRows;  // fewer rows per element: the row kernel
     // mixed forms on the tensor cores (tcgen05): tiles of 128 elements with identical
     // matrices, matrix operand images split into hi / lo parts
@@ -251,11 +252,26 @@ inline bool lane_forms_input(const hgg_handle *h) {
     return h->lane && !h->op.tensor && h->op.physics != HGG_PHYSICS_ADVECTION;
 }
 
+// every stage input has exactly one earlier vector, the previous one (explicit RK4, midpoint)
+inline bool chain_tableau(const hgg_handle *h) {
+    const int S = h->S;
+    for (int i = 1; i < S; ++i)
+        for (int j = 0; j < i; ++j)
+            if ((h->rk_a[i * S + j] != 0.0) != (j == i - 1)) return false;
+    return true;
+}
+// the stored-matrix tiles: each stage then forms the next one's input, one vector, which
+// the pipelined kernel can copy (a source term is added after the stage: not with one)
+inline bool lin_forms_input(const hgg_handle *h, bool in_batch) {
+    return h->d_lin_win[0] && !h->lane && !h->src && chain_tableau(h) &&
+           (in_batch || lin_pipe_wanted(h->lin_R, h->lin_tiles, h->num_sms));
+}
+
 // Inputs and outputs of stage i of one Runge-Kutta step from sol[from] into
 // sol[1 - from] (stages as in HpgemAPISimplified_Impl.h:788-820; zero tableau
 // entries are skipped).
 template <typename KT>
-StageIOT<KT> make_stage_io(const hgg_handle *h, int from, double dt, int i, int *status) {
+StageIOT<KT> make_stage_io(const hgg_handle *h, int from, double dt, int i, int *status, bool in_batch = false) {
     const int S = h->S;
     auto kv = [&](int j) { return static_cast<KT *>(h->k[j]); };
     StageIOT<KT> io{};
@@ -283,6 +299,13 @@ StageIOT<KT> make_stage_io(const hgg_handle *h, int from, double dt, int i, int 
             }
         }
         io.blast = dt * h->rk_b[S - 1];
+    }
+    if (lin_forms_input(h, in_batch)) {
+        if (i > 0) io.win = h->d_lin_win[(i - 1) & 1];
+        if (!last) {
+            io.wnext = h->d_lin_win[i & 1];
+            io.wcoef = dt * h->rk_a[(i + 1) * S + i];
+        }
     }
     if (lane_forms_input(h)) {
         if (i > 0) io.win = h->d_lane_win[(i - 1) & 1];

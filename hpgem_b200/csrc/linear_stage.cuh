@@ -215,7 +215,7 @@ __device__ __forceinline__ void linear_tile_body(const StageIOT<KT> &io, const L
             const int32_t e = tel[n];
             if (e < 0 || e >= io.n_elements || r >= rows) continue;
             const int64_t idx = (int64_t)e * R + r0 + r;
-            stage_output(io, idx, io.u[idx], Os[n * kLinOutStride + r]);
+            stage_output_few(io, idx, io.u[idx], Os[n * kLinOutStride + r]);
         }
     }
 }
@@ -224,6 +224,197 @@ template <typename KT>
 __global__ void __launch_bounds__(256) linear_tile_stage(const StageIOT<KT> io, const LinearGeom g,
                                                           const LinearTiles t) {
     linear_tile_body<KT>(io, g, t, blockIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// pipelined form of the tiles
+// ---------------------------------------------------------------------------
+// The products of linear_tile_body, in the same order (so the results are the same bit
+// for bit), where the stage input is one vector: the solution, or the input the previous
+// stage formed (io.win).  What bounds the tiles is the FP64 tensor pipe (64 FMAs per clock
+// and SM, the rate of the CUDA cores); the form above left it idle between its barriers
+// and for the 64-element tiles' last wave.  Here
+//   * a block of four warps takes 32 elements (half a tile): twice the blocks, and four or
+//     six of them share an SM (whole tiles per block: 3092 against 2586 us per RK4 step on
+//     64^3 hexahedra at p = 3);
+//   * the next chunk of 32 columns (matrix rows and gathered element rows) is copied
+//     asynchronously while this one's products run: one barrier per chunk, and no load's
+//     latency between barriers;
+//   * a warp forms 16 elements times four bands of eight rows (8 elements times four where
+//     an element has at most 32 rows), so six fragment loads feed eight products.
+// Measured, us per RK4 step: hexahedra at p = 3 24 x 20 x 28 290 -> 167, 64^3 2928 -> 2586
+// (23.3 TFLOP/s, 0.66 of cuBLAS DGEMM 8192^3); the wave on 12^3 x 5 tetrahedra at p = 2
+// 203 -> 114.
+constexpr int kLinPipeN = 32;
+constexpr int kLinPipeThreads = 128;
+__host__ __device__ constexpr int lin_pipe_rows(bool wide) { return wide ? kLinRows : 32; }  // rows per pass
+__host__ __device__ constexpr int lin_pipe_smem(bool wide) {
+    return 2 * (lin_pipe_rows(wide) + kLinPipeN) * kLinStride * (int)sizeof(double);
+}
+__host__ __device__ constexpr int lin_pipe_blocks(bool wide) { return wide ? 4 : 6; }  // per SM
+// Narrow elements take it only while all blocks run at once: triangles at p = 5, FP32 form,
+// 64^2 x 2 90 -> 66 us per RK4 step, but 128^2 x 2 115 (linear_tile_stage) and 135.
+inline bool lin_pipe_wanted(int R, int64_t tiles, int num_sms) { return R > 32 || 2 * tiles <= 6 * (int64_t)num_sms; }
+
+template <int BYTES>
+__device__ __forceinline__ void lin_copy(double *dst, const double *src, bool valid) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    const int n = valid ? BYTES : 0;  // the rest is filled with zeros
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+// WIDE: more than 32 rows per element.  PAIRS: an even number of rows (16-byte copies).
+// block: two per tile.
+template <typename KT, bool WIDE, bool PAIRS>
+__device__ __forceinline__ void linear_pipe_body(const StageIOT<KT> &io, const LinearGeom &g, const LinearTiles &t,
+                                                 int64_t block) {
+    constexpr int ROWS = lin_pipe_rows(WIDE), EL = kLinPipeN, NT = WIDE ? 2 : 1, BUF = (ROWS + EL) * kLinStride;
+    constexpr int PER = PAIRS ? 2 : 1, PARTS = kLinKC / PER;  // doubles per copy, copies per row
+    constexpr int STEP = kLinPipeThreads / PARTS;             // rows copied at once
+    extern __shared__ __align__(16) double lin_pipe_shared[];
+    const int R = g.R, S = g.slots;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+    const int n0 = WIDE ? (warp & 1) * (EL / 2) : warp * 8, b0 = WIDE ? (warp >> 1) * 4 : 0;  // the warp's elements, bands
+    const int64_t tile = block >> 1;
+    const int32_t *tel = t.elems + tile * kLinTileN + (block & 1) * EL;
+    const int32_t *mats = t.mats + tile * (S + 1);
+    const double *w = io.win ? io.win : io.u;
+    const int crow = tid / PARTS, ccol = (tid % PARTS) * PER;  // this thread's copies: rows crow + STEP i, column ccol
+    auto element = [&](int n) {  // of the block, -1: padding
+        const int32_t e = __ldg(tel + n);
+        return e >= 0 && e < io.n_elements ? e : -1;
+    };
+    int32_t el[EL / STEP];  // the elements whose rows this thread copies
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < EL / STEP; ++i) {
+        el[i] = element(crow + STEP * i);
+        any = any || el[i] >= 0;
+    }
+    if (!__syncthreads_or(any)) return;  // (a group's last tile: its second half may be empty)
+    // next slot with a matrix after s; S + 1 when there is none
+    auto next_slot = [&](int s) {
+        for (++s; s <= S; ++s) {
+            const int32_t m = __ldg(mats + s);
+            if (m >= g.n_mats && tid == 0) atomicOr(io.status, 4);
+            if (m >= 0 && m < g.n_mats) break;
+        }
+        return s;
+    };
+    int32_t src[EL / STEP];  // of the slot being copied
+    auto sources = [&](int s) {
+#pragma unroll
+        for (int i = 0; i < EL / STEP; ++i) {
+            int32_t se = el[i];
+            if (s > 0 && se >= 0) se = __ldg(g.nbr + (int64_t)se * S + (s - 1));
+            if (se >= io.n_elements || se < -1) {
+                atomicOr(io.status, 1);
+                se = -1;
+            }
+            src[i] = se;
+        }
+    };
+    for (int r0 = 0; r0 < R; r0 += ROWS) {
+        const int rows = min(ROWS, R - r0), rw = (rows + 7) & ~7;
+        auto copy = [&](int s, int kc, double *buf) {
+            const double *A = g.table_rm + (size_t)__ldg(mats + s) * R * R;
+            const bool in = kc + ccol < R;
+#pragma unroll
+            for (int i = 0; i < ROWS / STEP; ++i) {
+                const int r = crow + STEP * i;
+                if (r < rw) {
+                    const bool ok = in && r < rows;
+                    lin_copy<8 * PER>(buf + r * kLinStride + ccol, ok ? A + (size_t)(r0 + r) * R + kc + ccol : A, ok);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < EL / STEP; ++i) {
+                const bool ok = in && src[i] >= 0;
+                lin_copy<8 * PER>(buf + (ROWS + crow + STEP * i) * kLinStride + ccol,
+                                  ok ? w + (int64_t)src[i] * R + kc + ccol : w, ok);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        double acc[NT][4][2];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[n][b][0] = acc[n][b][1] = 0.0;
+        int s = next_slot(-1), kc = 0, at = 0;
+        if (s <= S) {
+            sources(s);
+            copy(s, 0, lin_pipe_shared);
+        }
+        while (s <= S) {
+            const double *As = lin_pipe_shared + at * BUF, *Bs = As + ROWS * kLinStride;
+            const int kmax = min(kLinKC, R - kc);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();  // this chunk is here, and the other buffer's products are done
+            at ^= 1;
+            kc += kLinKC;
+            if (kc >= R) {
+                kc = 0;
+                s = next_slot(s);
+                if (s <= S) sources(s);
+            }
+            if (s <= S) copy(s, kc, lin_pipe_shared + at * BUF);
+#pragma unroll 2
+            for (int k4 = 0; k4 < kmax; k4 += 4) {
+                double b[NT];
+#pragma unroll
+                for (int n = 0; n < NT; ++n) b[n] = Bs[(n0 + 8 * n + gid) * kLinStride + k4 + tig];
+#pragma unroll
+                for (int band = 0; band < 4; ++band) {
+                    if ((b0 + band) * 8 >= rows) continue;
+                    const double a = As[((b0 + band) * 8 + gid) * kLinStride + k4 + tig];
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) dmma_m8n8k4(acc[n][band][0], acc[n][band][1], a, b[n]);
+                }
+            }
+        }
+        __syncthreads();  // all products: stage the outputs as [element][row]
+        constexpr int OS = ROWS + 1;
+        double *Os = lin_pipe_shared;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int band = 0; band < 4; ++band)
+                if ((b0 + band) * 8 < rows) {
+                    const int e = n0 + 8 * n + tig * 2, r = (b0 + band) * 8 + gid;
+                    Os[e * OS + r] = acc[n][band][0];
+                    Os[(e + 1) * OS + r] = acc[n][band][1];
+                }
+        __syncthreads();
+#pragma unroll 4
+        for (int i = tid; i < EL * ROWS; i += kLinPipeThreads) {
+            const int n = i / ROWS, r = i % ROWS;
+            const int32_t e = element(n);
+            if (e < 0 || r >= rows) continue;
+            const int64_t idx = (int64_t)e * R + r0 + r;
+            stage_output_few(io, idx, io.u[idx], Os[n * OS + r]);
+        }
+        __syncthreads();  // the outputs are read (the next pass copies over them)
+    }
+}
+
+template <typename KT, bool WIDE, bool PAIRS>
+__global__ void __launch_bounds__(kLinPipeThreads, lin_pipe_blocks(WIDE))
+    linear_pipe_stage(const StageIOT<KT> io, const LinearGeom g, const LinearTiles t) {
+    linear_pipe_body<KT, WIDE, PAIRS>(io, g, t, blockIdx.x);
+}
+
+// calls f(WIDE, PAIRS) for elements of R rows and a stage input at `w` (a caller's vector
+// may start at any double: 16-byte copies only where it starts at 16 bytes)
+template <typename F>
+void lin_pipe_dispatch(int R, const double *w, F &&f) {
+    const bool pairs = R % 2 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
+    auto with = [&](auto wide) {
+        if (pairs) f(wide, std::true_type{});
+        else f(wide, std::false_type{});
+    };
+    if (R > 32) with(std::true_type{});
+    else with(std::false_type{});
 }
 
 }  // namespace hgg

@@ -119,6 +119,16 @@ int launch_linear(hgg_handle *h, const StageIOT<KT> &io) {
                  R, h->lin_slots, epb, h->lin_mats};
     if (h->lin_tiles > 0) {
         LinearTiles t{h->d_lin_tile_elems, h->d_lin_tile_mats};
+        if (lin_pipe_wanted(R, h->lin_tiles, h->num_sms) && (io.nin == 0 || io.win)) {  // one vector to read
+            lin_pipe_dispatch(R, io.win ? io.win : io.u, [&](auto wide, auto pairs) {
+                constexpr bool W = decltype(wide)::value, P = decltype(pairs)::value;
+                cudaFuncSetAttribute(linear_pipe_stage<KT, W, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     lin_pipe_smem(W));
+                linear_pipe_stage<KT, W, P>
+                    <<<(unsigned)(2 * h->lin_tiles), kLinPipeThreads, lin_pipe_smem(W), h->stream>>>(io, g, t);
+            });
+            return 0;
+        }
         linear_tile_stage<KT><<<(unsigned)h->lin_tiles, 256, 0, h->stream>>>(io, g, t);
         return 0;
     }
