@@ -14,7 +14,11 @@ namespace hgg {
 
 void invert_matrix(int n, const double *A, double *Ainv) {
     // Gauss-Jordan with partial pivoting on [A | I]
-    std::vector<double> M((size_t)n * 2 * n, 0.0);
+    double small[18];  // (element Jacobians: no allocation)
+    std::vector<double> large;
+    if (n > 3) large.resize((size_t)n * 2 * n);
+    double *M = n > 3 ? large.data() : small;
+    std::fill(M, M + (size_t)n * 2 * n, 0.0);
     for (int i = 0; i < n; ++i) {
         for (int j = 0; j < n; ++j) M[i * 2 * n + j] = A[i * n + j];
         M[i * 2 * n + n + i] = 1.0;
@@ -357,13 +361,16 @@ HostOperators build_operators(const hgg_problem_desc &desc, bool faces) {
     }
 
     // face operators per (test tabulation, trial tabulation) pair
-    std::map<std::pair<int, int>, int> pair_id;
+    // (a table where it is small, as for the few tabulations of a mesh, else a map)
+    const size_t nt = (size_t)std::max(desc.n_face_tabs, 0);
+    std::vector<int> pair_table(nt <= 256 ? nt * nt : 0, -1);
+    std::map<std::pair<int, int>, int> pair_map;
+    int n_pairs = 0;
     auto get_pair = [&](int s, int n) {
-        auto key = std::make_pair(s, n);
-        auto it = pair_id.find(key);
-        if (it != pair_id.end()) return it->second;
-        int id = (int)pair_id.size();
-        pair_id.emplace(key, id);
+        int &known = pair_table.empty() ? pair_map.emplace(std::make_pair(s, n), -1).first->second
+                                        : pair_table[(size_t)s * nt + n];
+        if (known >= 0) return known;
+        const int id = known = n_pairs++;
         std::vector<double> E((size_t)nB * nB, 0.0);
         const double *ps = desc.face_tabs + (size_t)s * nQf * nB;
         const double *pn = desc.face_tabs + (size_t)n * nQf * nB;
@@ -432,7 +439,7 @@ HostOperators build_operators(const hgg_problem_desc &desc, bool faces) {
     }
     for (size_t s = 0; s < slots; ++s)
         if (op.nbr[s] < 0) throw std::invalid_argument("element face without a neighbour");
-    op.n_pairs = (int)pair_id.size();
+    op.n_pairs = n_pairs;
     op.tensor = try_tensor(desc, op);
     return op;
 }

@@ -2,13 +2,11 @@
 #include "setup.h"
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
 #include <sstream>
 #include <stdexcept>
-#include <unordered_map>
 
 namespace hgg {
 
@@ -180,25 +178,6 @@ StructuredDescription parse_structured(const std::string &text) {
     return d;
 }
 
-namespace {
-
-struct FaceKey {
-    std::array<int64_t, 4> v;
-    bool operator==(const FaceKey &o) const { return v == o.v; }
-};
-struct FaceKeyHash {
-    size_t operator()(const FaceKey &k) const {
-        uint64_t h = 1469598103934665603ull;
-        for (int64_t x : k.v) {
-            h ^= (uint64_t)x + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
-            h *= 1099511628211ull;
-        }
-        return (size_t)h;
-    }
-};
-
-}  // namespace
-
 Mesh structured_mesh(const StructuredDescription &d) {
     const int dim = (int)d.n.size();
     std::vector<int64_t> n_elem(d.n), n_nodes(dim);
@@ -299,25 +278,46 @@ void pair_faces(Mesh &m) {
     const ShapeInfo &si = shape_info(m.shape);
     const int dim = m.dim;
     const int fv = dim == 1 ? 1 : si.face_vertices;
-    std::unordered_map<FaceKey, int64_t, FaceKeyHash> open;
-    open.reserve((size_t)(m.n_elements * si.n_faces / 2 + 16));
+    // open addressing by the hash of the sorted nodes; a face stays in the table when it is
+    // paired and is passed over from then on (a map of nodes took half of the set-up)
+    const size_t faces = (size_t)m.n_elements * si.n_faces;
+    size_t cap = 16;
+    while (cap < faces + faces / 4) cap <<= 1;
+    std::vector<int32_t> table(cap, -1);
+    std::vector<int64_t> keys;  // [face][fv] sorted nodes
+    keys.reserve((faces / 2 + 16) * fv);
+    m.face_elements.reserve(faces + 32);
+    m.face_local.reserve(faces + 32);
+    m.face_perm.reserve((faces / 2 + 16) * fv);
     for (int64_t e = 0; e < m.n_elements; ++e) {
         for (int f = 0; f < si.n_faces; ++f) {
-            FaceKey key{{-1, -1, -1, -1}};
-            int64_t g[4];
-            for (int k = 0; k < fv; ++k) g[k] = key.v[k] = m.nodes[e * m.n_vertices + si.faces[f][k]];
-            std::sort(key.v.begin(), key.v.begin() + fv);
-            auto it = open.find(key);
-            if (it == open.end()) {
-                open.emplace(key, m.n_faces());
+            int64_t g[4], key[4];
+            for (int k = 0; k < fv; ++k) g[k] = key[k] = m.nodes[e * m.n_vertices + si.faces[f][k]];
+            std::sort(key, key + fv);
+            uint64_t hash = 0;
+            for (int k = 0; k < fv; ++k) {
+                hash = (hash ^ (uint64_t)key[k]) * 0x9E3779B97F4A7C15ull;
+                hash ^= hash >> 29;
+            }
+            size_t at = hash & (cap - 1);
+            int64_t fid = -1;
+            for (; table[at] >= 0; at = (at + 1) & (cap - 1)) {
+                const int64_t t = table[at];
+                if (m.face_elements[2 * t + 1] < 0 && std::equal(key, key + fv, &keys[t * fv])) {
+                    fid = t;
+                    break;
+                }
+            }
+            if (fid < 0) {
+                if (m.n_faces() >= INT32_MAX) throw std::invalid_argument("too many faces");
+                table[at] = (int32_t)m.n_faces();
+                keys.insert(keys.end(), key, key + fv);
                 m.face_elements.push_back(e);
                 m.face_elements.push_back(-1);
                 m.face_local.push_back(f);
                 m.face_local.push_back(-1);
                 for (int k = 0; k < fv; ++k) m.face_perm.push_back(-1);
             } else {
-                int64_t fid = it->second;
-                open.erase(it);
                 int64_t L = m.face_elements[2 * fid];
                 int fL = m.face_local[2 * fid];
                 m.face_elements[2 * fid + 1] = e;
@@ -587,12 +587,13 @@ StructuredProblem build_problem(Mesh mesh, int order, int physics, const double 
     // face tabulations: one per (local face, vertex order) that occurs
     const int fv = d == 1 ? 1 : si.face_vertices;
     const int nQf = P.face_rule.size();
-    std::map<std::vector<int>, int> tabs;
+    std::vector<int> tab_ids(8 * 8 * 8 * 8, -1);  // by the local vertices (at most four, below 8)
+    int n_tabs = 0;
     auto tab_of = [&](const std::vector<int> &verts) {
-        auto it = tabs.find(verts);
-        if (it != tabs.end()) return it->second;
-        int id = (int)tabs.size();
-        tabs.emplace(verts, id);
+        int code = 0;
+        for (int v : verts) code = 8 * code + v;
+        if (tab_ids[code] >= 0) return tab_ids[code];
+        const int id = tab_ids[code] = n_tabs++;
         for (int q = 0; q < nQf; ++q) {
             double xi[3];
             face_to_element(m.shape, verts.data(), &P.face_rule.points[q * (d - 1)], xi);
@@ -611,6 +612,17 @@ StructuredProblem build_problem(Mesh mesh, int order, int physics, const double 
         for (int k = 0; k < fs.n_vertices; ++k)
             for (int c = 0; c < d - 1; ++c) fcentre[c] += fs.vertices[k][c] / fs.n_vertices;
     }
+    double tangent[6][2][3];  // of every local face's map, in the reference element
+    for (int f = 0; f < si.n_faces && d > 1; ++f)
+        for (int c = 0; c < d - 1; ++c) {
+            double a[3], b[3], xp[3] = {fcentre[0], fcentre[1], fcentre[2]};
+            double xm[3] = {fcentre[0], fcentre[1], fcentre[2]};
+            xp[c] += 0.5;
+            xm[c] -= 0.5;
+            face_to_element(m.shape, si.faces[f], xp, a);
+            face_to_element(m.shape, si.faces[f], xm, b);
+            for (int k = 0; k < d; ++k) tangent[f][c][k] = a[k] - b[k];
+        }
     for (int64_t f = 0; f < F; ++f) {
         int64_t L = m.face_elements[2 * f];
         int fL = m.face_local[2 * f], fR = m.face_local[2 * f + 1];
@@ -628,19 +640,12 @@ StructuredProblem build_problem(Mesh mesh, int order, int physics, const double 
         double n[3] = {1.0, 0.0, 0.0};
         if (d > 1) {
             double T[3][2];
-            for (int c = 0; c < d - 1; ++c) {
-                double a[3], b[3], xp[3] = {fcentre[0], fcentre[1], fcentre[2]};
-                double xm[3] = {fcentre[0], fcentre[1], fcentre[2]};
-                xp[c] += 0.5;
-                xm[c] -= 0.5;
-                face_to_element(m.shape, si.faces[fL], xp, a);
-                face_to_element(m.shape, si.faces[fL], xm, b);
+            for (int c = 0; c < d - 1; ++c)
                 for (int r = 0; r < d; ++r) {
                     double s = 0.0;
-                    for (int k = 0; k < d; ++k) s += J[r * d + k] * (a[k] - b[k]);
+                    for (int k = 0; k < d; ++k) s += J[r * d + k] * tangent[fL][c][k];
                     T[r][c] = s;
                 }
-            }
             if (d == 2) {
                 n[0] = T[1][0];
                 n[1] = -T[0][0];
@@ -659,7 +664,7 @@ StructuredProblem build_problem(Mesh mesh, int order, int physics, const double 
         for (int c = 0; c < d; ++c) dot += n[c] * (fc[c] - ec[c]);
         for (int c = 0; c < d; ++c) P.normals[f * d + c] = dot < 0 ? -n[c] : n[c];
     }
-    P.n_face_tabs = (int)tabs.size();
+    P.n_face_tabs = n_tabs;
     return P;
 }
 
