@@ -17,21 +17,24 @@ int launch_slice(hgg_handle *h, const StageIOT<KT> &io) {
     for (int sd = 0; sd < 2; ++sd)
         for (int a = 0; a < 4; ++a) sops.L[sd][a] = op.lift[sd * 4 + a];
     const int64_t blocks = (op.nE + SliceShape::TE - 1) / SliceShape::TE;
-    const dim3 grid((unsigned)blocks), block(SliceShape::THREADS);
     const bool fin = io.unew != nullptr;
     // each block asks L2 for the inputs of the tile a block of the next resident wave runs
     // (5 blocks per SM resident): measured 4 % faster per RK4 step for the FP32 form and
     // 2-3 % for the FP64 form's first three stages; the FP64 final stage (4 resident
     // blocks, three more input vectors) measured slower with it and goes without
     const int64_t ahead = (sizeof(KT) == 4 || !io.unew) ? (int64_t)h->num_sms * 5 : 0;
+    auto launch = [&](auto kern) {
+        const double *geo = h->d_slice_geo;
+        launch_chained(kern, (unsigned)blocks, SliceShape::THREADS, 0, h->stream, io, geo, sops, ahead);
+    };
     if (io.nin == 0 && (!fin || io.nfin == 0))
-        tensor_slice<KT, 0, 0><<<grid, block, 0, h->stream>>>(io, h->d_slice_geo, sops, ahead);
+        launch(tensor_slice<KT, 0, 0>);
     else if (io.nin == 1 && (!fin || io.nfin == 0))
-        tensor_slice<KT, 1, 0><<<grid, block, 0, h->stream>>>(io, h->d_slice_geo, sops, ahead);
+        launch(tensor_slice<KT, 1, 0>);
     else if (io.nin == 1 && fin && io.nfin == 3)
-        tensor_slice<KT, 1, 3><<<grid, block, 0, h->stream>>>(io, h->d_slice_geo, sops, ahead);
+        launch(tensor_slice<KT, 1, 3>);
     else
-        tensor_slice<KT, -1, -1><<<grid, block, 0, h->stream>>>(io, h->d_slice_geo, sops, ahead);
+        launch(tensor_slice<KT, -1, -1>);
     return 0;
 }
 
