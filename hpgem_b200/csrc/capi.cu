@@ -442,7 +442,18 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
     h->tensor_layout = op.tensor;
     h->slice_ok = op.tensor && op.dim == 3 && op.order == 3 && op.trace_pos[0] == 0 && op.trace_pos[1] == 1;
     std::vector<int32_t> lane_nbr;
-    h->lane_ok = h->lane = !h->slice_ok && tensor_lane_setup(op, h->tlane, lane_nbr);
+    // In the FP32 form a stage that reads many vectors (Dormand-Prince) is a long chain of
+    // loads for a thread with a whole element of 16 or more functions: below a warp or so
+    // per SM the one-shot kernel's thread per coefficient is faster (per step 32 x 45 p = 5
+    // 33 against 44 us, 60^2 p = 4 33 against 43; 100 x 90 p = 5 64 against 53)
+    int vectors = 0;
+    for (int i = 0; i < h->S; ++i) {
+        int n = 0;
+        for (int j = 0; j < i; ++j) n += h->rk_a[i * h->S + j] != 0.0;
+        vectors = std::max(vectors, n);
+    }
+    const bool one_shot = h->mixed && vectors > 2 && op.nB >= 16 && op.nE < 185 * 32;
+    h->lane_ok = h->lane = !h->slice_ok && !one_shot && tensor_lane_setup(op, h->tlane, lane_nbr);
     LaneMesh lmesh;
     LaneTables ltab;
     if (!op.tensor && !linear && desc->precision != HGG_PRECISION_BF16X3) lane_setup(h, lmesh, ltab);
@@ -1113,6 +1124,31 @@ __global__ void sum_pairs(const double *a, const double *b, int64_t n, double *p
     }
 }
 
+// the partials' sums (as sum_pairs) and the status word, for one copy to the host
+__global__ void finish_sums(const double *a, const double *b, int64_t n, const int *status, double *out) {
+    __shared__ double sa[kSumThreads], sb[kSumThreads];
+    double x = 0.0, y = 0.0;
+    for (int64_t i = threadIdx.x; i < n; i += kSumThreads) {
+        x += a[i];
+        y += b[i];
+    }
+    sa[threadIdx.x] = x;
+    sb[threadIdx.x] = y;
+    __syncthreads();
+    for (int w = kSumThreads / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+            sa[threadIdx.x] += sa[threadIdx.x + w];
+            sb[threadIdx.x] += sb[threadIdx.x + w];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[0] = sa[0];
+        out[1] = sb[0];
+        out[2] = (double)*status;
+    }
+}
+
 // undo a rejected step: u -= dt b_j k_j for j = 0..S-1, one update after the other as
 // the reference's scaleAndAddVector calls do (HpgemAPISimplified_Impl.h:843-848)
 template <typename KT>
@@ -1138,8 +1174,9 @@ ErrStages<KT> err_stages(const hgg_handle *h, double dt, const std::vector<doubl
     return ks;
 }
 
-// error and solution norm of the step just taken (sol[cur] is the updated solution)
-int error_and_norm(hgg_handle *h, double dt, double *error, double *norm) {
+// error and solution norm of the step just taken (sol[cur] is the updated solution), and
+// the status word after it: one copy and one wait for the three
+int error_and_norm(hgg_handle *h, double dt, double *error, double *norm, int *status) {
     const int64_t nE = h->op.nE;
     const int nb = h->op.V * h->op.nB;
     double *err2 = h->d_reduce, *nrm = h->d_reduce + nE;
@@ -1153,15 +1190,15 @@ int error_and_norm(hgg_handle *h, double dt, double *error, double *norm) {
     const int parts = 256;
     double *pa = h->d_reduce + 2 * nE, *pb = pa + parts;
     sum_pairs<<<parts, kSumThreads, 0, h->stream>>>(err2, nrm, nE, pa, pb);
-    sum_pairs<<<1, kSumThreads, 0, h->stream>>>(pa, pb, parts, pa + 2 * parts, pb + 2 * parts);
+    finish_sums<<<1, kSumThreads, 0, h->stream>>>(pa, pb, parts, h->d_status, pa + 2 * parts);
     h->launches += 3;
     HGG_CUDA(h, cudaGetLastError());
-    double out[2];
-    HGG_CUDA(h, cudaMemcpyAsync(&out[0], pa + 2 * parts, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    HGG_CUDA(h, cudaMemcpyAsync(&out[1], pb + 2 * parts, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    double out[3];
+    HGG_CUDA(h, cudaMemcpyAsync(out, pa + 2 * parts, sizeof(out), cudaMemcpyDeviceToHost, h->stream));
     HGG_CUDA(h, cudaStreamSynchronize(h->stream));
     *error = std::sqrt(out[0]);
     *norm = out[1];
+    *status = (int)out[2];
     return 0;
 }
 
@@ -1191,7 +1228,7 @@ int hgg_step_adaptive(hgg_handle *h, double *time, double max_relative_error, do
     h->store_last = true;
     double dt = std::min(*dt_estimate, dt_max);
     double error = std::numeric_limits<double>::infinity(), norm = 0.0;
-    int rej = 0;
+    int rej = 0, status = 0;
     int rc = 0;
     while (max_relative_error * norm < error || std::isinf(error)) {
         const int from = h->cur;
@@ -1199,7 +1236,7 @@ int hgg_step_adaptive(hgg_handle *h, double *time, double max_relative_error, do
         if (!rc) rc = enqueue_step(h, from, dt);
         if (rc) break;
         h->cur = 1 - from;
-        rc = error_and_norm(h, dt, &error, &norm);
+        rc = error_and_norm(h, dt, &error, &norm, &status);
         if (rc) break;
         if (max_relative_error * norm < error || std::isinf(error)) {
             const unsigned grid = 4 * h->num_sms;
@@ -1224,7 +1261,7 @@ int hgg_step_adaptive(hgg_handle *h, double *time, double max_relative_error, do
     *time += dt;
     if (dt_taken) *dt_taken = dt;
     if (rejections) *rejections = rej;
-    return check_status(h);
+    return status ? fail(h, HGG_ERR_DEVICE, status_message(status)) : 0;
 }
 
 }  // extern "C"
