@@ -175,8 +175,9 @@ int64_t hgg_vector_length(const hgg_handle *h);
 /* 1 when the sum-factorised tensor-product kernel drives this handle,
  * 0 when the dense reference-operator kernel does, 2 for the stored-matrix
  * kernels: handles from hgg_create_linear*, and matrix-free handles whose
- * operator the library folded into per-element matrices because the grouped
- * tensor-core kernel applies them faster (advection on triangles, p >= 4);
+ * operator the library folded into per-element matrices (advection on
+ * triangles, p >= 4; structured meshes step them on the lane kernels, see
+ * hgg_set_kernel_variant);
  * 3 for the same stored-matrix tiles on the fifth-generation tensor cores
  * (tcgen05: the FP32-mixed form as three TF32 products, the split-BF16 form as
  * three BF16 products, 128-element tiles). */
@@ -191,13 +192,17 @@ int hgg_set_store_last_stage(hgg_handle *h, int32_t enable);
  * device; NULL restores the handle's own stream). */
 int hgg_set_stream(hgg_handle *h, void *stream);
 
-/* Selects the kernel organisation: 0 (default) automatic; on the
- * sum-factorised path 1 is one block per small group of elements and 2 the
- * pipelined kernel; on the dense path 1 runs one thread per element row and 2
- * the grouped kernel (tiles of elements with equal operators) wherever the
- * mesh has such tiles, whatever the contraction type (automatic takes it for
- * the wave with FP64 contractions).  All compute the same result; the choice
- * exists for comparison and profiling.
+/* Selects the kernel organisation: 0 (default) automatic, which on structured
+ * meshes takes the lane kernels (one element per thread, vectors in tiles of 32
+ * elements: advection on quadrilaterals, hexahedra of order 1 and 2 and
+ * simplices, the wave up to 36 basis functions); on the sum-factorised path 1
+ * is one block per small group of elements and 2 the pipelined kernel; on the
+ * dense path 1 runs one thread per element row and 2 the grouped kernel (tiles
+ * of elements with equal operators) wherever the mesh has such tiles, whatever
+ * the contraction type.  Changing it moves the handle's vectors to the other
+ * kernel's layout; their values stay.  All compute the same result (the FP32
+ * form's lane kernels bit for bit what the automatic choice among the others
+ * gives); the choice exists for comparison and profiling.
  * Hexahedra of order 3 keep their vectors in a tiled layout that only their
  * slice kernel reads: any variant but 0 returns HGG_ERR_UNSUPPORTED there. */
 int hgg_set_kernel_variant(hgg_handle *h, int32_t variant);
@@ -471,7 +476,8 @@ void *hgg_batch_stream(const hgg_batch *b);
 
 /* Kernel class i (0 .. hgg_batch_num_classes - 1, classes with members):
  * info10 = kind (0 matrix-free dense, 1 sum-factorised, 2 sum-factorised slices,
- * 3 stored-matrix tiles, 4 tensor-core tiles), shape, dim, order, physics,
+ * 3 stored-matrix tiles, 4 tensor-core tiles, 5 wave tiles, 6 sum-factorised
+ * lanes, 7 lanes of simplices and the wave), shape, dim, order, physics,
  * precision (0 FP64, 1 FP32-mixed, 2 split-BF16), stages, members, elements,
  * coefficients. */
 int hgg_batch_class_info(const hgg_batch *b, int32_t i, int64_t *info10);
