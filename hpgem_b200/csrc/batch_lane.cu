@@ -72,7 +72,7 @@ void launch(const LaneClassStage &c, Kern kern, const Item *items, int threads, 
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) == cudaSuccess) *c.occupancy = n;
         return;
     }
-    launch_chained(kern, c.grid, threads, smem, c.stream, items, c.n, c.total, c.parity, c.remaining);
+    launch_chained(true, kern, c.grid, threads, smem, c.stream, items, c.n, c.total, c.parity, c.remaining);
 }
 
 template <typename KT>

@@ -989,6 +989,13 @@ int hgg_test_arm_without_copy(hgg_handle *h, int32_t polls) {
     return 0;
 }
 
+int hgg_test_set_overlap(hgg_handle *h, int32_t enable) {
+    if (!h) return fail(h, HGG_ERR_INVALID, "null handle");
+    if (h->overlap != (enable != 0)) release_graphs(h);
+    h->overlap = enable != 0;
+    return 0;
+}
+
 // ---- right-hand side without allocation ---------------------------------------
 // The sum-factorised handles keep their vectors in tensor order on the device,
 // so a right-hand side of caller-owned vectors in hpGEM order needs two

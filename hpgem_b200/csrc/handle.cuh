@@ -75,6 +75,7 @@ struct hgg_handle {
     // one-element-per-thread kernels (lane = element, tiled layout): the handle has one, and
     // its vectors are in that kernel's layout (kernel variant 0)
     bool lane_ok = false, lane = false;
+    bool overlap = true;                  // chained launches start early (hgg_test_set_overlap)
     hgg::TensorLaneGeom tlane{};          // sum-factorised handles
     hgg::LaneGeom lgeo{};                  // simplices and the wave
     double *d_lane_win[2] = {nullptr, nullptr};  // ... the wave: stage inputs formed ahead (contraction type)
@@ -169,18 +170,19 @@ void release_graphs(hgg_handle *h);
 // device vector into `staging` (pinned, h->N_alloc doubles), the layout change on the host
 int solution_to_host(hgg_handle *h, double *staging, double *out);
 
-// Launch of a stage kernel that calls chain_next and chain_wait: its start overlaps the
-// previous kernel's end on the same stream (anything else before it is waited for in
+// Launch of a stage kernel that calls chain_next and chain_wait: with `overlap` its start
+// overlaps the previous kernel's end on the same stream (anything else before it is waited for in
 // full), which takes most of the gap between two stages out.  Per RK4 step: 32^2
 // quadrilaterals at p = 2 12.7 -> 9.1 us, triangles 192 x 160 at p = 3 22.6 -> 17.9, the
 // FP32 wave on 14 x 18 x 12 x 5 tetrahedra at p = 3 160 -> 154.  (Letting the next stage
 // start at a kernel's beginning instead of before its outputs spreads its blocks unevenly
 // over the SMs: the triangles took 23.7.)
 template <typename... K, typename... A>
-void launch_chained(void (*kern)(K...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, A &&...args) {
+void launch_chained(bool overlap, void (*kern)(K...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
+                    A &&...args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    attr.val.programmaticStreamSerializationAllowed = overlap;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);

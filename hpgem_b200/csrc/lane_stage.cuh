@@ -131,7 +131,7 @@ __device__ __forceinline__ void lane_output(const StageIOT<KT> &io, int64_t idx,
 #pragma unroll
     for (int f = 0; f < F; ++f)
 #pragma unroll
-        for (int i = 0; i < RB; ++i) r[f][i] = i < rows ? ldg_f64(u + f * step + 32 * i) : 0.0;
+        for (int i = 0; i < RB; ++i) r[f][i] = i < rows ? load_coef(u + f * step + 32 * i) : 0.0;
 #pragma unroll 1
     for (int j = 0; j < io.nfin; ++j) {
         const double bj = io.bfin[j];
@@ -140,7 +140,7 @@ __device__ __forceinline__ void lane_output(const StageIOT<KT> &io, int64_t idx,
         for (int f = 0; f < F; ++f)
 #pragma unroll
             for (int i = 0; i < RB; ++i)
-                if (i < rows) r[f][i] += bj * ldg_k(kj + f * step + 32 * i);
+                if (i < rows) r[f][i] += bj * load_coef(kj + f * step + 32 * i);
     }
     if (io.wnext) {
         CT *out = reinterpret_cast<CT *>(io.wnext) + idx;
@@ -567,7 +567,7 @@ __device__ __forceinline__ void advection_lane_body(const StageIOT<KT> &io, cons
     auto input = [&](int64_t from, int count, auto offset, CT *x) {
         double v[CH];
 #pragma unroll
-        for (int i = 0; i < CH; ++i) v[i] = i < count ? ldg_f64(io.u + from + offset(i)) : 0.0;
+        for (int i = 0; i < CH; ++i) v[i] = i < count ? load_coef(io.u + from + offset(i)) : 0.0;
         if (NIN != 0) {
             const int nin = NIN > 0 ? NIN : io.nin;
 #pragma unroll 1
@@ -576,7 +576,7 @@ __device__ __forceinline__ void advection_lane_body(const StageIOT<KT> &io, cons
                 const KT *kj = io.kin[j] + from;
 #pragma unroll
                 for (int i = 0; i < CH; ++i)
-                    if (i < count) v[i] += cj * ldg_k(kj + offset(i));
+                    if (i < count) v[i] += cj * load_coef(kj + offset(i));
             }
         }
 #pragma unroll

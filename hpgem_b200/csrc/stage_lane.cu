@@ -10,7 +10,7 @@ namespace {
 template <typename Kern, typename KT>
 void launch(hgg_handle *h, Kern kern, const StageIOT<KT> &io, int threads, int smem) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    launch_chained(kern, (unsigned)h->lgeo.n_chunks, threads, smem, h->stream, io, h->lgeo);
+    launch_chained(h->overlap, kern, (unsigned)h->lgeo.n_chunks, threads, smem, h->stream, io, h->lgeo);
 }
 
 template <typename KT, int DIM, int NFL, int WAVE>

@@ -25,7 +25,7 @@ int launch_slice(hgg_handle *h, const StageIOT<KT> &io) {
     const int64_t ahead = (sizeof(KT) == 4 || !io.unew) ? (int64_t)h->num_sms * 5 : 0;
     auto launch = [&](auto kern) {
         const double *geo = h->d_slice_geo;
-        launch_chained(kern, (unsigned)blocks, SliceShape::THREADS, 0, h->stream, io, geo, sops, ahead);
+        launch_chained(h->overlap, kern, (unsigned)blocks, SliceShape::THREADS, 0, h->stream, io, geo, sops, ahead);
     };
     if (io.nin == 0 && (!fin || io.nfin == 0))
         launch(tensor_slice<KT, 0, 0>);
@@ -49,6 +49,7 @@ int launch_tensor_lane(hgg_handle *h, const StageIOT<KT> &io) {
     const bool ok = tensor_lane_dispatch(h->op.dim, h->op.order, [&](auto p, auto d) {
         lane_stage_shape(io.nin, io.unew != nullptr, [&](auto nin, auto fin) {
             launch_chained(
+                h->overlap,
                 tensor_lane<KT, decltype(p)::value, decltype(d)::value, decltype(nin)::value, decltype(fin)::value>, blocks,
                 32 * warps, 0, h->stream, io, g);
         });

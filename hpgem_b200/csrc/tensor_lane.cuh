@@ -55,7 +55,7 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
         constexpr int N = decltype(count)::value;
         double v[N];
 #pragma unroll
-        for (int i = 0; i < N; ++i) v[i] = ldg_f64(io.u + from + 32 * pos(i));
+        for (int i = 0; i < N; ++i) v[i] = load_coef(io.u + from + 32 * pos(i));
         if (NIN != 0) {
             const int nin = NIN > 0 ? NIN : io.nin;
 #pragma unroll 1
@@ -63,7 +63,7 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
                 const double cj = io.cin[j];
                 const KT *kj = io.kin[j] + from;
 #pragma unroll
-                for (int i = 0; i < N; ++i) v[i] += cj * ldg_k(kj + 32 * pos(i));
+                for (int i = 0; i < N; ++i) v[i] += cj * load_coef(kj + 32 * pos(i));
             }
         }
 #pragma unroll
@@ -96,12 +96,12 @@ __device__ __forceinline__ void tensor_lane_body(const StageIOT<KT> &io, const T
     double fu[FIN ? NB : 1];
     if (FIN) {
 #pragma unroll
-        for (int i = 0; i < NB; ++i) fu[i] = ldg_f64(io.u + base + 32 * i);
+        for (int i = 0; i < NB; ++i) fu[i] = load_coef(io.u + base + 32 * i);
         for (int j = 0; j < io.nfin; ++j) {
             const double bj = io.bfin[j];
             const KT *kj = io.kfin[j] + base;
 #pragma unroll
-            for (int i = 0; i < NB; ++i) fu[i] += bj * ldg_k(kj + 32 * i);
+            for (int i = 0; i < NB; ++i) fu[i] += bj * load_coef(kj + 32 * i);
         }
     }
     // FP32 form: the rounded fluxes of every face

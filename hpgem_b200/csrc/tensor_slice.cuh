@@ -60,19 +60,19 @@ __device__ __forceinline__ int64_t tiled_index(int64_t n, int j) {
     return (n >> 5) * SliceShape::TILE + j * 32 + (n & 31);
 }
 
+// an entry of a table no kernel writes (geometry): the non-coherent path
 __device__ __forceinline__ double ldg_f64(const double *p) {
     double v;
     asm("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
 
-__device__ __forceinline__ float ldg_f32(const float *p) {
-    float v;
-    asm("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ldg_k(const double *p) { return ldg_f64(p); }
-__device__ __forceinline__ double ldg_k(const float *p) { return (double)ldg_f32(p); }
+// A coefficient of the solution or of a stage vector.  A chained stage is already resident
+// while the previous one writes these, and non-coherent loads are defined only for memory
+// that nobody writes while the kernel lives; nor would an asm without a memory clobber stay
+// behind chain_wait.  A plain load is coherent and does.
+__device__ __forceinline__ double load_coef(const double *p) { return *p; }
+__device__ __forceinline__ double load_coef(const float *p) { return (double)*p; }
 
 template <typename CT>
 __device__ __forceinline__ CT slice_flux(int md, CT sg, CT self, CT nbr) {
@@ -129,18 +129,21 @@ __device__ __forceinline__ void tensor_slice_body(const StageIOT<KT> &io, const 
     if (prefetch_ahead > 0 && threadIdx.x == 0 && tile + prefetch_ahead < n_tiles)
         prefetch_tile(io, geo, tile + prefetch_ahead, nin, nfin);
     for (int i = threadIdx.x; i < TE * GR; i += SliceShape::THREADS) G[i] = ldg_f64(geo + t0 * GR + i);
-    if constexpr (CHAINED) chain_wait();
+    if constexpr (CHAINED) {
+        chain_wait();
+        chain_next();  // (after the wait: never more than two stages resident)
+    }
     CT w[16];
     {
         double wd[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) wd[i] = ldg_f64(io.u + base + 32 * (i + 16 * c));
+        for (int i = 0; i < 16; ++i) wd[i] = load_coef(io.u + base + 32 * (i + 16 * c));
 #pragma unroll
         for (int jj = 0; jj < nin; ++jj) {
             const double cj = io.cin[jj];
             const KT *kj = io.kin[jj] + base;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) wd[i] += cj * ldg_k(kj + 32 * (i + 16 * c));
+            for (int i = 0; i < 16; ++i) wd[i] += cj * load_coef(kj + 32 * (i + 16 * c));
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) w[i] = (CT)wd[i];
@@ -187,12 +190,12 @@ __device__ __forceinline__ void tensor_slice_body(const StageIOT<KT> &io, const 
                 const int64_t nbase = ((int64_t)n >> 5) * TILE + (n & 31);
                 double v[8];
 #pragma unroll
-                for (int q = 0; q < nq; ++q) v[q] = ldg_f64(io.u + nbase + 32 * nbr_pos(s, q));
+                for (int q = 0; q < nq; ++q) v[q] = load_coef(io.u + nbase + 32 * nbr_pos(s, q));
 #pragma unroll
                 for (int jj = 0; jj < nin; ++jj) {
                     const double cj = io.cin[jj];
 #pragma unroll
-                    for (int q = 0; q < nq; ++q) v[q] += cj * ldg_k(io.kin[jj] + nbase + 32 * nbr_pos(s, q));
+                    for (int q = 0; q < nq; ++q) v[q] += cj * load_coef(io.kin[jj] + nbase + 32 * nbr_pos(s, q));
                 }
 #pragma unroll
                 for (int q = 0; q < nq; ++q) NB[f][q] = (CT)v[q];
@@ -224,13 +227,13 @@ __device__ __forceinline__ void tensor_slice_body(const StageIOT<KT> &io, const 
     double fu[16];
     if (io.unew) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) fu[i] = ldg_f64(io.u + base + 32 * (i + 16 * c));
+        for (int i = 0; i < 16; ++i) fu[i] = load_coef(io.u + base + 32 * (i + 16 * c));
 #pragma unroll
         for (int jj = 0; jj < nfin; ++jj) {
             const double bj = io.bfin[jj];
             const KT *kj = io.kfin[jj] + base;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) fu[i] += bj * ldg_k(kj + 32 * (i + 16 * c));
+            for (int i = 0; i < 16; ++i) fu[i] += bj * load_coef(kj + 32 * (i + 16 * c));
         }
     }
     const CT ax = (CT)g[0], ay = (CT)g[1], az = (CT)g[2];
@@ -279,7 +282,6 @@ __device__ __forceinline__ void tensor_slice_body(const StageIOT<KT> &io, const 
 template <typename KT, int NIN, int NFIN>
 __global__ void __launch_bounds__(SliceShape::THREADS, sizeof(KT) == 4 ? 5 : (NFIN == 0 ? 5 : 4))
     tensor_slice(const StageIOT<KT> io, const double *__restrict__ geo, const SliceOps op, int64_t prefetch_ahead) {
-    chain_next();
     tensor_slice_body<KT, NIN, NFIN, true>(io, geo, op, blockIdx.x, prefetch_ahead, gridDim.x);
 }
 

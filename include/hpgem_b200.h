@@ -270,6 +270,12 @@ int64_t hgg_launch_count(const hgg_handle *h);
  * HGG_ERR_UNSUPPORTED on handles of other kernels. */
 int hgg_test_arm_without_copy(hgg_handle *h, int32_t polls);
 
+/* For the tests: enable = 0 makes every stage of this handle start when the one
+ * before it has ended.  By default the slice kernel and the lane kernels are
+ * launched so that a stage's blocks may be resident while the previous stage's
+ * last blocks run; the results are the same. */
+int hgg_test_set_overlap(hgg_handle *h, int32_t enable);
+
 /* ---- stand-alone set-up: hpGEM's host side, restated ------------------- */
 
 /* Builds the descriptor hpGEM would build from a Preprocessor "structured"
