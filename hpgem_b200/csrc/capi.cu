@@ -371,7 +371,7 @@ int alloc_tile_inputs(hgg_handle *h) {
 }
 
 // Lane kernel of simplices and of the wave: the mesh's groups, their tables (host).
-void lane_setup(hgg_handle *h, LaneMesh &m, LaneTables &t) {
+void lane_setup(hgg_handle *h, const hgg_problem_desc &desc, LaneMesh &m, LaneTables &t) {
     const HostOperators &op = h->op;
     const bool wave = op.physics != HGG_PHYSICS_ADVECTION;
     if (!lane_size(op.dim, op.nfl, wave, op.nB) || op.nB != lane_basis(op.dim, op.nfl, op.order)) return;
@@ -389,7 +389,7 @@ void lane_setup(hgg_handle *h, LaneMesh &m, LaneTables &t) {
     // a server's estimate of a handle's footprint leaves 320 bytes per element and 4 MB, and
     // the FP32 wave's stage inputs are half of what it counts
     const int spare = 320 + (wave && elem_bytes == 4 ? 8 * op.V * op.nB : 0);
-    if (!lane_mesh(op, h->lane_tiles, folded, bytes, spare, m)) return;
+    if (!lane_mesh(desc, op, h->lane_tiles, folded, bytes, spare, m)) return;
     if (!(wave ? lane_wave_tables(op, m, folded, elem_bytes, t)
                 : lane_advection_tables(op, m, folded, elem_bytes, t))) return;
     if (t.group_bytes > 96 * 1024) return;
@@ -453,10 +453,10 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
         vectors = std::max(vectors, n);
     }
     const bool one_shot = h->mixed && vectors > 2 && op.nB >= 16 && op.nE < 185 * 32;
-    h->lane_ok = h->lane = !h->slice_ok && !one_shot && tensor_lane_setup(op, h->tlane, lane_nbr);
+    h->lane_ok = h->lane = !h->slice_ok && !one_shot && tensor_lane_setup(*desc, op, h->mixed, h->tlane, lane_nbr);
     LaneMesh lmesh;
     LaneTables ltab;
-    if (!op.tensor && !linear && desc->precision != HGG_PRECISION_BF16X3) lane_setup(h, lmesh, ltab);
+    if (!op.tensor && !linear && desc->precision != HGG_PRECISION_BF16X3) lane_setup(h, *desc, lmesh, ltab);
     h->tiled = h->slice_ok || h->lane;
     if (h->slice_ok) h->tile_elems = SliceShape::TE;
     if (h->mixed && !mixed_supported(h))

@@ -4,25 +4,140 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <optional>
+
+#include "refshapes.h"
 
 namespace hgg {
 
-bool tensor_lane_setup(const HostOperators &op, TensorLaneGeom &g, std::vector<int32_t> &nbr) {
+// The extent of the mesh along each axis bounds its coordinates' magnitude (a box that lies
+// within a few times its own size of the origin, as meshes do).  The descriptor has no
+// coordinates: the elements' places follow from their Jacobians, face by face, breadth
+// first, so that periodic images stay within one period of the start.
+GeometryRounding::GeometryRounding(const hgg_problem_desc &dsc, const HostOperators &o) : desc(dsc), op(o) {
+    const int d = op.dim, nf = op.nfl;
+    const ShapeInfo &si = shape_info(op.shape);
+    const int fv = d == 1 ? 1 : si.face_vertices;
+    double centre[3] = {0.0, 0.0, 0.0}, to_face[6][3] = {};  // face centres seen from the element's
+    for (int k = 0; k < si.n_vertices; ++k)
+        for (int c = 0; c < d; ++c) centre[c] += si.vertices[k][c] / si.n_vertices;
+    for (int f = 0; f < nf; ++f)
+        for (int c = 0; c < d; ++c) {
+            for (int k = 0; k < fv; ++k) to_face[f][c] += si.vertices[si.faces[f][k]][c] / fv;
+            to_face[f][c] -= centre[c];
+        }
+    std::vector<int8_t> other((size_t)op.nE * nf, 0);  // the neighbour's local face
+    for (int64_t f = 0; f < desc.n_faces; ++f)
+        for (int s = 0; s < 2; ++s)
+            other[desc.face_elements[2 * f + s] * nf + desc.face_local[2 * f + s]] = (int8_t)desc.face_local[2 * f + 1 - s];
+    std::vector<double> place((size_t)op.nE * d, 0.0);
+    std::vector<uint8_t> seen(op.nE, 0);
+    std::vector<int32_t> queue;
+    queue.reserve(op.nE);
+    double lo[3] = {0.0, 0.0, 0.0}, hi[3] = {0.0, 0.0, 0.0};
+    for (int64_t start = 0; start < op.nE; ++start) {
+        if (seen[start]) continue;
+        seen[start] = 1;
+        queue.push_back((int32_t)start);
+        for (size_t at = queue.size() - 1; at < queue.size(); ++at) {
+            const int64_t e = queue[at];
+            const double *J = desc.jacobians + e * d * d, *x = &place[e * d];
+            for (int r = 0; r < d; ++r) {
+                double half = 0.0;  // (an element lies within |J_rc| of its centre, summed over c)
+                for (int c = 0; c < d; ++c) half += std::fabs(J[r * d + c]);
+                lo[r] = std::min(lo[r], x[r] - half);
+                hi[r] = std::max(hi[r], x[r] + half);
+            }
+            for (int f = 0; f < nf; ++f) {
+                const int32_t n = op.nbr[e * nf + f];
+                if (seen[n]) continue;
+                seen[n] = 1;
+                const double *Jn = desc.jacobians + (int64_t)n * d * d;
+                const double *a = to_face[f], *b = to_face[other[e * nf + f]];
+                for (int r = 0; r < d; ++r) {
+                    double y = x[r];
+                    for (int c = 0; c < d; ++c) y += J[r * d + c] * a[c] - Jn[r * d + c] * b[c];
+                    place[(int64_t)n * d + r] = y;
+                }
+                queue.push_back(n);
+            }
+        }
+    }
+    // a coordinate is off by half a unit in the last place (2^-54 of [0, L]'s upper half, twice
+    // that where the box starts at L), a difference of two by twice as much, and two
+    // elements' differences by four times
+    for (int r = 0; r < d; ++r) eps[r] = 0x1p-51 * (hi[r] - lo[r]);
+}
+
+// With J' = J + dJ, |dJ_kl| <= eps_k, the inverse changes by J^{-1} dJ J^{-1}.  The rest is
+// linear in it: ahat = J^{-1} a, G = J^{-T}, and n / |J| = J^{-T} m with m the reference
+// element's face normal (Nanson's formula).
+std::vector<double> GeometryRounding::bounds(int64_t e) const {
+    const int d = op.dim, nf = op.nfl;
+    const bool wave = op.physics != HGG_PHYSICS_ADVECTION;
+    const ShapeInfo &si = shape_info(op.shape);
+    double inv[9], t[9];  // J^{-1}, the bound of its change
+    invert_matrix(d, desc.jacobians + e * d * d, inv);
+    for (int c = 0; c < d; ++c)
+        for (int r = 0; r < d; ++r) {
+            double rows = 0.0, columns = 0.0;
+            for (int k = 0; k < d; ++k) {
+                rows += std::fabs(inv[c * d + k]) * eps[k];
+                columns += std::fabs(inv[k * d + r]);
+            }
+            t[c * d + r] = rows * columns;
+        }
+    std::vector<double> out;
+    double along[3] = {0.0, 0.0, 0.0};  // ... of ahat
+    for (int c = 0; c < d; ++c)
+        for (int r = 0; r < d; ++r) along[c] += t[c * d + r] * std::fabs(desc.advection[r]);
+    if (wave)
+        for (int r = 0; r < d; ++r)
+            for (int c = 0; c < d; ++c) out.push_back(t[c * d + r]);
+    else out.insert(out.end(), along, along + d);
+    for (int f = 0; f < nf; ++f) {
+        const int *v = si.faces[f];
+        double m[3] = {1.0, 0.0, 0.0};
+        if (d == 2) {
+            m[0] = 0.5 * (si.vertices[v[1]][1] - si.vertices[v[0]][1]);
+            m[1] = 0.5 * (si.vertices[v[1]][0] - si.vertices[v[0]][0]);
+        } else if (d == 3) {
+            const double scale = si.face_vertices == 4 ? 0.25 : 1.0;  // reference faces of area 4 and 1/2
+            for (int c = 0; c < 3; ++c) {
+                const int i = (c + 1) % 3, j = (c + 2) % 3;
+                const double *x = si.vertices[v[0]], *y = si.vertices[v[1]], *z = si.vertices[v[2]];
+                m[c] = scale * ((y[i] - x[i]) * (z[j] - x[j]) - (y[j] - x[j]) * (z[i] - x[i]));
+            }
+        }
+        double sigma = 0.0;
+        for (int c = 0; c < d; ++c) sigma += std::fabs(m[c]) * along[c];
+        if (!wave) out.push_back(sigma);
+        for (int r = 0; r < d && wave; ++r) {
+            double nu = 0.0;
+            for (int c = 0; c < d; ++c) nu += 0.5 * std::fabs(m[c]) * t[c * d + r];
+            out.push_back(nu);
+        }
+    }
+    return out;
+}
+
+bool tensor_lane_setup(const hgg_problem_desc &desc, const HostOperators &op, bool fp32, TensorLaneGeom &g,
+                       std::vector<int32_t> &nbr) {
     const int d = op.dim, np = op.np, ns = 2 * d;
     if (!op.tensor || !tensor_lane_order(d, op.order) || np != op.order + 1) return false;
     if (op.trace_pos[0] != 0 || op.trace_pos[1] != 1) return false;
     const double *a0 = op.elem_geo.data(), *s0 = op.t_sigma.data();
     const int8_t *m0 = op.t_mode.data();
-    double abig = 0.0, sbig = 0.0;
-    for (int c = 0; c < d; ++c) abig = std::max(abig, std::fabs(a0[c]));
-    for (int s = 0; s < ns; ++s) sbig = std::max(sbig, std::fabs(s0[s]));
-    const double atol = std::ldexp(abig, -40), stol = std::ldexp(sbig, -40);
-    if (!std::isfinite(abig) || !std::isfinite(sbig)) return false;
+    // (a hypercube's sigma is +-ahat of its axis: the same bound)
+    const std::vector<double> bound = GeometryRounding(desc, op).bounds(0);
+    auto equal = [&](double v, double v0, int axis) {
+        return std::isfinite(v) && std::fabs(v - v0) <= bound[axis] && (!fp32 || (float)v == (float)v0);
+    };
     for (int64_t e = 0; e < op.nE; ++e) {
         for (int c = 0; c < d; ++c)
-            if (!(std::fabs(op.elem_geo[e * d + c] - a0[c]) <= atol)) return false;
+            if (!equal(op.elem_geo[e * d + c], a0[c], c)) return false;
         for (int s = 0; s < ns; ++s)
-            if (op.t_mode[e * ns + s] != m0[s] || !(std::fabs(op.t_sigma[e * ns + s] - s0[s]) <= stol)) return false;
+            if (op.t_mode[e * ns + s] != m0[s] || !equal(op.t_sigma[e * ns + s], s0[s], s / 2)) return false;
     }
     g = TensorLaneGeom{};
     for (int i = 0; i < np * np; ++i) g.D1[i] = (float)op.D1[i];
@@ -91,14 +206,16 @@ std::vector<int32_t> same_pairs(const HostOperators &op) {
 
 }  // namespace
 
-bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int coefficient_bytes, int spare_bytes, LaneMesh &m) {
+bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_tiles_max, bool folded,
+               int coefficient_bytes, int spare_bytes, LaneMesh &m) {
     const int nf = op.nfl, d = op.dim, R = op.V * op.nB;
     const bool wave = op.physics != 0;
     // (plain tables hold no geometry: their kernels read every element's own)
     const int eg = !folded ? 0 : wave ? d * d : d, fg = !folded ? 0 : wave ? d : 1;
-    // group key: pair operators, upwind modes, and the geometry rounded to 2^-40 of its
-    // largest entry (only the key is rounded; a group steps with its first element's
-    // values, which differ from the others' by the rounding of vertex coordinates).
+    // A group: elements with the same pair operators and upwind modes whose geometry differs
+    // from the first one's by no more than the rounding of vertex coordinates, entry by
+    // entry; all of them step with that one's values.  The hash key has the operators, the
+    // modes, and the geometry rounded to 2^-20 of its largest entry (a filter only).
     // (the plain tables' results depend on their operators' last bits: no merging there)
     std::vector<int32_t> same;
     if (folded) same = same_pairs(op);
@@ -116,8 +233,8 @@ bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int co
         if (!std::isfinite(big)) return false;
         int e = 0;
         std::frexp(big, &e);
-        // adding 1.5 * 2^52 rounds to a whole number (the scaled values are below 2^40)
-        const double scale = big > 0.0 ? std::ldexp(1.0, 40 - e) : 0.0, magic = 0x1.8p52;
+        // adding 1.5 * 2^52 rounds to a whole number (the scaled values are below 2^20)
+        const double scale = big > 0.0 ? std::ldexp(1.0, 20 - e) : 0.0, magic = 0x1.8p52;
         for (int i = 0; i < n; ++i) {
             const volatile double r = v[i] * scale + magic;
             const double q = r;
@@ -127,6 +244,20 @@ bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int co
         return true;
     };
     const size_t most = (size_t)op.nE / 10 + 296;  // more groups than this take too much padding
+    std::optional<GeometryRounding> rounding;
+    if (folded) rounding.emplace(desc, op);
+    std::vector<double> bounds;  // [group][eg + nf fg]
+    const int ng = eg + nf * fg;
+    auto equal = [&](int64_t e, int32_t g) {
+        const int64_t r = m.representative[g];
+        const double *b = &bounds[(size_t)g * ng];
+        bool same_geo = true;
+        for (int i = 0; i < eg; ++i) same_geo &= std::fabs(op.elem_geo[e * eg + i] - op.elem_geo[r * eg + i]) <= b[i];
+        for (int i = 0; i < nf * fg; ++i)
+            same_geo &= std::fabs(op.face_geo[e * nf * fg + i] - op.face_geo[r * nf * fg + i]) <= b[eg + i];
+        return same_geo;
+    };
+    const int most_alike = 64;  // groups of one key: elements that vary by less than the filter sees
     for (int64_t e = 0; e < op.nE; ++e) {
         uint64_t *k = key.data();
         for (int f = 0; f < nf; ++f) {
@@ -140,13 +271,20 @@ bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int co
             hash ^= hash >> 29;
         }
         size_t at = hash & (table.size() - 1);
-        while (table[at] >= 0 && !std::equal(key.begin(), key.end(), keys.begin() + (size_t)table[at] * words))
-            at = (at + 1) & (table.size() - 1);
+        for (int alike = 0; table[at] >= 0; at = (at + 1) & (table.size() - 1)) {
+            if (!std::equal(key.begin(), key.end(), keys.begin() + (size_t)table[at] * words)) continue;
+            if (!folded || equal(e, table[at])) break;
+            if (++alike >= most_alike) return false;
+        }
         if (table[at] < 0) {
             if (count.size() >= most || count.size() * 2 >= table.size()) return false;
             table[at] = (int32_t)count.size();
             keys.insert(keys.end(), key.begin(), key.end());
             m.representative.push_back(e);
+            if (folded) {
+                const std::vector<double> b = rounding->bounds(e);
+                bounds.insert(bounds.end(), b.begin(), b.end());
+            }
             count.push_back(0);
         }
         group[e] = table[at];

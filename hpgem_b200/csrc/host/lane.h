@@ -35,11 +35,29 @@ struct TensorLaneGeom {
 // orders with a kernel: every coefficient of an element fits a thread's registers
 inline bool tensor_lane_order(int dim, int p) { return (dim == 2 && p >= 1 && p <= 5) || (dim == 3 && p >= 1 && p <= 2); }
 
+// How much rounding of the vertex coordinates can change an element's geometry.  The cells
+// of a structured mesh are equal up to that, and only up to that may an element step with
+// another one's values: each entry is compared with its own bound, which on flat cells is
+// far below the largest entry's rounding.
+class GeometryRounding {
+  public:
+    GeometryRounding(const hgg_problem_desc &desc, const HostOperators &op);
+    // bounds for element e: of its elem_geo, then of its face_geo
+    std::vector<double> bounds(int64_t e) const;
+
+  private:
+    const hgg_problem_desc &desc;
+    const HostOperators &op;
+    double eps[3] = {0.0, 0.0, 0.0};  // of a difference of coordinates along each axis
+};
+
 // Fills g (but for the device pointer) and nbr when the mesh qualifies: a sum-factorised
-// handle of an order with a kernel, whose elements agree in ahat, sigma and upwind modes
-// to 2^-40 of the largest entry (the cells of a structured mesh differ by the rounding of
-// their vertex coordinates; all of them then step with the first element's values).
-bool tensor_lane_setup(const HostOperators &op, TensorLaneGeom &g, std::vector<int32_t> &nbr);
+// handle of an order with a kernel, whose elements have equal upwind modes and ahat and
+// sigma equal up to the coordinates' rounding (all of them then step with the first
+// element's values); in the FP32 form, equal as that form rounds them, so that its results
+// are the general kernels'.
+bool tensor_lane_setup(const hgg_problem_desc &desc, const HostOperators &op, bool fp32, TensorLaneGeom &g,
+                       std::vector<int32_t> &nbr);
 
 // ---- simplices and the wave (lane_stage.cuh) -------------------------------------
 // Elements with the same operators and geometry (a few groups on a structured mesh) are
@@ -94,7 +112,8 @@ struct LaneTables {
 // (unstructured meshes, very small ones).
 // coefficient_bytes: of all vectors of the handle, per coefficient; spare_bytes: what the
 // padding may take per element (and 4 MB).
-bool lane_mesh(const HostOperators &op, int chunk_tiles_max, bool folded, int coefficient_bytes, int spare_bytes, LaneMesh &m);
+bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_tiles_max, bool folded,
+               int coefficient_bytes, int spare_bytes, LaneMesh &m);
 // Tables of the groups: `folded` as described in lane_stage.cuh, or plain with entries of
 // elem_bytes; false when the operators
 // do not have the sparsity it relies on (a face couples more functions than its trace
