@@ -180,32 +180,6 @@ bool tensor_lane_setup(const hgg_problem_desc &desc, const HostOperators &op, bo
 
 // ---- simplices and the wave -------------------------------------------------------
 
-namespace {
-
-// The first pair operator equal to each one.  A face's points are numbered from its left
-// element, so one operator appears once per numbering; the copies differ by rounding.
-std::vector<int32_t> same_pairs(const HostOperators &op) {
-    const size_t nn = (size_t)op.nB * op.nB;
-    std::vector<int32_t> same(op.n_pairs);
-    for (int p = 0; p < op.n_pairs; ++p) {
-        const double *A = &op.pairs[p * nn];
-        double big = 0.0;
-        for (size_t i = 0; i < nn; ++i) big = std::max(big, std::fabs(A[i]));
-        same[p] = p;
-        for (int q = 0; q < p && same[p] == p; ++q) {
-            if (same[q] != q) continue;
-            const double *B = &op.pairs[q * nn];
-            bool eq = std::equal(&op.pair_trace[(size_t)p * op.nB], &op.pair_trace[(size_t)(p + 1) * op.nB],
-                                 &op.pair_trace[(size_t)q * op.nB]);
-            for (size_t i = 0; i < nn && eq; ++i) eq = std::fabs(A[i] - B[i]) <= 0x1p-40 * big;
-            if (eq) same[p] = q;
-        }
-    }
-    return same;
-}
-
-}  // namespace
-
 bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_tiles_max, bool folded,
                int coefficient_bytes, int spare_bytes, LaneMesh &m) {
     const int nf = op.nfl, d = op.dim, R = op.V * op.nB;
@@ -217,10 +191,9 @@ bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_
     // entry; all of them step with that one's values.  The hash key has the operators, the
     // modes, and the geometry rounded to 2^-20 of its largest entry (a filter only).
     // (the plain tables' results depend on their operators' last bits: no merging there)
-    std::vector<int32_t> same;
-    if (folded) same = same_pairs(op);
-    else
-        for (int p = 0; p < op.n_pairs; ++p) same.push_back(p);
+    std::vector<int32_t> same = op.pair_same;
+    if (!folded)
+        for (int p = 0; p < op.n_pairs; ++p) same[p] = p;
     m = LaneMesh{};
     std::vector<int32_t> group(op.nE);
     std::vector<int64_t> count;

@@ -39,6 +39,7 @@ struct HostOperators {
     std::vector<double> pairs;      // [n_pairs][nB][nB]
     int n_pairs = 0;
     std::vector<uint8_t> pair_trace;  // [n_pairs][nB] whether the trial side's function does not vanish on the face
+    std::vector<int32_t> pair_same;   // [n_pairs] the first one with the same face matrix (up to rounding)
     std::vector<int32_t> nbr;       // [E][nfl]
     std::vector<int32_t> self_pair; // [E][nfl]
     std::vector<int32_t> nbr_pair;  // [E][nfl]
