@@ -302,6 +302,7 @@ struct hgg_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr;
     std::vector<hgg_handle *> handles;  // by slot, nullptr when free
+    std::vector<std::shared_ptr<int>> membership;  // by slot: the handle's count of batches
     std::vector<double> dt;
     std::vector<int> base;               // the handle's current buffer when it was added
     std::vector<int> cls;                // class index of each slot
@@ -1004,6 +1005,8 @@ void destroy_batch(hgg_batch *b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     release_batch_graph(b);
+    for (auto &m : b->membership)
+        if (m) --*m;
     for (auto &c : b->classes) {
         if (c.stream) cudaStreamSynchronize(c.stream);
         for (void *p : c.d_items) cudaFreeAsync(p, b->stream);
@@ -1034,6 +1037,8 @@ int remove_member(hgg_batch *b, int slot, int parity) {
     c.slots.erase(std::find(c.slots.begin(), c.slots.end(), slot));
     c.table_dirty = true;
     b->handles[slot] = nullptr;
+    --*b->membership[slot];
+    b->membership[slot].reset();
     b->cls[slot] = -1;
     b->remaining_host[slot] = 0;
     b->item_cache[slot].clear();
@@ -1056,6 +1061,7 @@ int hgg_batch_create(int32_t capacity, hgg_batch **out) {
     auto *b = new hgg_batch();
     b->cap = capacity;
     b->handles.assign(capacity, nullptr);
+    b->membership.assign(capacity, nullptr);
     b->dt.assign(capacity, 0.0);
     b->base.assign(capacity, 0);
     b->cls.assign(capacity, -1);
@@ -1166,6 +1172,8 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
     b->classes[ci].table_dirty = true;
     b->item_cache[free_slot].clear();  // formed at the next table upload
     b->handles[free_slot] = h;
+    b->membership[free_slot] = h->memberships;
+    ++*h->memberships;
     b->dt[free_slot] = dt;
     b->base[free_slot] = h->cur;
     b->cls[free_slot] = ci;
@@ -1184,7 +1192,10 @@ int hgg_batch_remove(hgg_batch *b, int32_t slot) {
     if (!b || slot < 0 || slot >= b->cap || !b->handles[slot]) return bfail(b, HGG_ERR_INVALID, "bad slot");
     int rc = read_counters(b);
     if (rc) return rc;
-    return remove_member(b, slot, b->parity_host[slot]);
+    hgg_handle *h = b->handles[slot];
+    if ((rc = remove_member(b, slot, b->parity_host[slot]))) return rc;
+    if (settle_layout(h)) return bfail(b, HGG_ERR_CUDA, hgg_last_error(h));
+    return 0;
 }
 
 int hgg_batch_step(hgg_batch *b, int32_t nsteps) {

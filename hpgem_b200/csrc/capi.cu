@@ -159,6 +159,13 @@ int set_lane_layout(hgg_handle *h, bool lane) {
     return 0;
 }
 
+int settle_layout(hgg_handle *h) {
+    const bool lane = h->lane_ok && h->variant == 0;
+    if (lane == h->lane || *h->memberships > 0) return 0;
+    release_graphs(h);
+    return set_lane_layout(h, lane);
+}
+
 int launch_stage(hgg_handle *h, const StageIO &io) {
     int rc;
     if (h->lane && !h->op.tensor) rc = launch_stage_lane(h, io);
@@ -971,14 +978,12 @@ int hgg_set_kernel_variant(hgg_handle *h, int32_t variant) {
     if (!h || variant < 0 || variant > 2) return fail(h, HGG_ERR_INVALID, "variant must be 0..2");
     if (variant != 0 && h->slice_ok)
         return fail(h, HGG_ERR_UNSUPPORTED, "hexahedra of order 3 have one kernel organisation (the slice kernel)");
-    if (variant != h->variant) {
-        release_graphs(h);
-        int rc;
-        const bool lane = h->lane_ok && variant == 0;
-        if (lane != h->lane && (rc = set_lane_layout(h, lane))) return rc;
-        h->variant = variant;
-    }
-    return 0;
+    const int was = h->variant;
+    if (variant != was) release_graphs(h);
+    h->variant = variant;
+    const int rc = settle_layout(h);
+    if (rc) h->variant = was;
+    return rc;
 }
 
 int hgg_test_arm_without_copy(hgg_handle *h, int32_t polls) {

@@ -75,6 +75,10 @@ struct hgg_handle {
     // one-element-per-thread kernels (lane = element, tiled layout): the handle has one, and
     // its vectors are in that kernel's layout (kernel variant 0)
     bool lane_ok = false, lane = false;
+    // batches that have the handle as a member: their tables hold its vectors' layout, so a
+    // change of the variant moves them when the last has let go (shared with the batch,
+    // which may outlive the handle)
+    std::shared_ptr<int> memberships = std::make_shared<int>(0);
     bool overlap = true;                  // chained launches start early (hgg_test_set_overlap)
     hgg::TensorLaneGeom tlane{};          // sum-factorised handles
     hgg::LaneGeom lgeo{};                  // simplices and the wave
@@ -166,6 +170,8 @@ inline int coefficients(const hgg_handle *h) { return h->op.V * h->op.nB; }
 // the automatic choice where it measured faster than the per-row kernel
 bool group_wave_wanted(const hgg_handle *h);
 void release_graphs(hgg_handle *h);
+// the vectors into the layout of the kernel variant, unless a batch steps them
+int settle_layout(hgg_handle *h);
 // the current solution in hpGEM order with no kernel on the device: one copy of the
 // device vector into `staging` (pinned, h->N_alloc doubles), the layout change on the host
 int solution_to_host(hgg_handle *h, double *staging, double *out);

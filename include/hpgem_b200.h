@@ -202,7 +202,9 @@ int hgg_set_stream(hgg_handle *h, void *stream);
  * the contraction type.  Changing it moves the handle's vectors to the other
  * kernel's layout; their values stay.  All compute the same result (the FP32
  * form's lane kernels bit for bit what the automatic choice among the others
- * gives); the choice exists for comparison and profiling.
+ * gives); the choice exists for comparison and profiling.  A batch steps its
+ * members with the kernels it took them in with; the vectors of a member move
+ * when it is removed.
  * Hexahedra of order 3 keep their vectors in a tiled layout that only their
  * slice kernel reads: any variant but 0 returns HGG_ERR_UNSUPPORTED there. */
 int hgg_set_kernel_variant(hgg_handle *h, int32_t variant);

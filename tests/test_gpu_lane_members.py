@@ -1,0 +1,66 @@
+"""GPU: the kernel variant of a handle that is a member of a batch.  The batch steps the
+member with the kernel it took it in with, whatever the variant is set to meanwhile, and the
+handle's own steps after it has left use the variant that was set.  Both organisations
+evaluate the same operator: 1e-12 of the largest coefficient, as in the lane tests."""
+import numpy as np
+import pytest
+
+import hpgem_b200
+
+from lane_helpers import kernel_class
+
+pytestmark = pytest.mark.gpu
+
+
+def make(cells, tri, order, physics):
+    d = len(cells)
+    if physics == "advection":
+        s = hpgem_b200.Advection(d, order, [0.7, -0.4, 0.5][:d], tableau="RK4_4")
+    else:
+        s = hpgem_b200.AcousticWave(d, order, c_inv=0.8, tableau="RK4_4", flux="upwind")
+    s.readMesh(hpgem_b200.structured_description(cells, [0.0] * d, [1.0] * d, tri, True))
+    s.handle.set_state(0, np.random.default_rng(3).standard_normal(s.handle.vector_length))
+    return s
+
+
+@pytest.mark.parametrize("cells,tri,order,physics", [([13, 9], False, 3, "advection"), ([24, 20], True, 3, "advection"),
+                                                     ([24, 20], True, 4, "advection"), ([8, 8, 8], True, 2, "wave")])
+@pytest.mark.parametrize("variants", [(0, 1), (0, 2), (1, 0)])
+def test_variant_set_on_a_member(cells, tri, order, physics, variants):
+    dt = 0.01 / max(cells) / (2 * order + 1) ** 2
+    ref = make(cells, tri, order, physics)
+    ref.handle.step(0.0, dt, 12)
+    want = ref.handle.get_state(0)
+    s = make(cells, tri, order, physics)
+    s.handle.set_kernel_variant(variants[0])
+    batch = hpgem_b200.Batch(2)
+    slot = batch.add(s, dt, 9)
+    batch.step(3)
+    s.handle.set_kernel_variant(variants[1])  # (the steps may still run)
+    batch.step(3)
+    batch.synchronize()
+    s.handle.set_kernel_variant(variants[0])
+    s.handle.set_kernel_variant(variants[1])
+    batch.step(3)
+    batch.synchronize()
+    assert batch.remaining(slot) == 0
+    batch.remove(slot)
+    batch.close()
+    assert (kernel_class(s) in ("lane tables", "sum-factorised lanes")) == (variants[1] == 0)
+    s.handle.step(0.0, dt, 3)
+    got = s.handle.get_state(0)
+    assert np.abs(got - want).max() / np.abs(want).max() < 1e-12
+
+
+def test_batch_closed_with_a_member():
+    s = make([24, 20], True, 3, "advection")
+    batch = hpgem_b200.Batch(1)
+    batch.add(s, 1e-5, 2)
+    batch.step(2)
+    batch.synchronize()
+    s.handle.set_kernel_variant(1)
+    batch.close()
+    s.handle.step(0.0, 1e-5, 2)
+    ref = make([24, 20], True, 3, "advection")
+    ref.handle.step(0.0, 1e-5, 4)
+    assert np.abs(s.handle.get_state(0) - ref.handle.get_state(0)).max() < 1e-12 * np.abs(ref.handle.get_state(0)).max()
