@@ -269,10 +269,11 @@ inline bool chain_tableau(const hgg_handle *h) {
     return true;
 }
 // the stored-matrix tiles: each stage then forms the next one's input, one vector, which
-// the pipelined kernel can copy (a source term is added after the stage: not with one)
+// the pipelined kernel can copy (a source term is added after the stage: not with one; a
+// batch steps its members without their sources, and with its class's kernel)
 inline bool lin_forms_input(const hgg_handle *h, bool in_batch) {
-    return h->d_lin_win[0] && !h->lane && !h->src && chain_tableau(h) &&
-           (in_batch || lin_pipe_wanted(h->lin_R, h->lin_tiles, h->num_sms));
+    return h->d_lin_win[0] && !h->lane && chain_tableau(h) &&
+           (in_batch || (!h->src && lin_pipe_wanted(h->lin_R, h->lin_tiles, h->num_sms)));
 }
 
 // Inputs and outputs of stage i of one Runge-Kutta step from sol[from] into

@@ -64,3 +64,24 @@ def test_batch_closed_with_a_member():
     ref = make([24, 20], True, 3, "advection")
     ref.handle.step(0.0, 1e-5, 4)
     assert np.abs(s.handle.get_state(0) - ref.handle.get_state(0)).max() < 1e-12 * np.abs(ref.handle.get_state(0)).max()
+
+
+def test_source_set_on_a_stored_matrix_member():
+    """A batch steps its members without source terms (it takes no handle that has one), also
+    a member that is given one later."""
+    d = hpgem_b200.structured_description([5, 4, 6], [0.0] * 3, [1.0] * 3, False, True)
+    solvers = [hpgem_b200.HpgemAPILinear(3, 2, "advection", advection=[0.7, -0.4, 0.5], tableau="RK4_4").readMesh(d)
+               for _ in range(2)]
+    u0 = np.random.default_rng(4).standard_normal(solvers[0].handle.vector_length)
+    for s in solvers:
+        s.handle.set_state(0, u0)
+    batch = hpgem_b200.Batch(1)
+    slot = batch.add(solvers[0], 1e-4, 3)
+    solvers[0].setSourceTerm(lambda x, t: np.ones(len(x)))
+    batch.step(3)
+    batch.synchronize()
+    batch.remove(slot)
+    batch.close()
+    solvers[1].handle.step(0.0, 1e-4, 3)
+    want = solvers[1].handle.get_state(0)
+    assert np.abs(solvers[0].handle.get_state(0) - want).max() < 1e-12 * np.abs(want).max()
