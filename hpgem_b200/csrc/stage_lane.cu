@@ -7,9 +7,11 @@ namespace hgg {
 
 namespace {
 
+// most: of a block of the kernel on any mesh.  The limit is the process's, so it is set to
+// that: a smaller mesh's launch on another thread does not lower it.
 template <typename Kern, typename KT>
-void launch(hgg_handle *h, Kern kern, const StageIOT<KT> &io, int threads, int smem) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+void launch(hgg_handle *h, Kern kern, const StageIOT<KT> &io, int threads, int smem, int most) {
+    if (most > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     launch_chained(h->overlap, kern, (unsigned)h->lgeo.n_chunks, threads, smem, h->stream, io, h->lgeo);
 }
 
@@ -21,18 +23,22 @@ int launch_lane(hgg_handle *h, const StageIOT<KT> &io) {
         using CT = DenseCT<KT, NB>;
         if constexpr (lane_size(DIM, NFL, WAVE, NB)) {
             if constexpr (WAVE) {
-                const int threads = 32 * LaneShape<KT, CT, DIM, NFL, NB, true>::RW * h->lane_tiles;
+                using SH = LaneShape<KT, CT, DIM, NFL, NB, true>;
+                const int threads = 32 * SH::RW * h->lane_tiles, bytes = h->lgeo.group_bytes;
                 if (io.win)
                     launch(h, wave_lane<KT, CT, CT, DIM, NFL, NB>, io, threads,
-                           wave_lane_smem<KT, CT, CT, DIM, NFL, NB>(h->lgeo.group_bytes, h->lane_tiles));
+                           wave_lane_smem<KT, CT, CT, DIM, NFL, NB>(bytes, h->lane_tiles),
+                           wave_lane_smem<KT, CT, CT, DIM, NFL, NB>(bytes, SH::TILES));
                 else
                     launch(h, wave_lane<KT, CT, double, DIM, NFL, NB>, io, threads,
-                           wave_lane_smem<KT, CT, double, DIM, NFL, NB>(h->lgeo.group_bytes, h->lane_tiles));
+                           wave_lane_smem<KT, CT, double, DIM, NFL, NB>(bytes, h->lane_tiles),
+                           wave_lane_smem<KT, CT, double, DIM, NFL, NB>(bytes, SH::TILES));
             } else {
                 const int threads = 32 * LaneShape<KT, CT, DIM, NFL, NB, false>::RW * h->lane_tiles;
-                if (io.nin == 0) launch(h, advection_lane<KT, CT, DIM, NFL, NB, 0>, io, threads, h->lgeo.group_bytes);
-                else if (io.nin == 1) launch(h, advection_lane<KT, CT, DIM, NFL, NB, 1>, io, threads, h->lgeo.group_bytes);
-                else launch(h, advection_lane<KT, CT, DIM, NFL, NB, -1>, io, threads, h->lgeo.group_bytes);
+                const int bytes = h->lgeo.group_bytes;  // the same on every mesh
+                if (io.nin == 0) launch(h, advection_lane<KT, CT, DIM, NFL, NB, 0>, io, threads, bytes, bytes);
+                else if (io.nin == 1) launch(h, advection_lane<KT, CT, DIM, NFL, NB, 1>, io, threads, bytes, bytes);
+                else launch(h, advection_lane<KT, CT, DIM, NFL, NB, -1>, io, threads, bytes, bytes);
             }
             done = true;
         }
