@@ -297,7 +297,9 @@ bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_
         for (int64_t i = 0; i < n; ++i) m.slot[members[p.group][p.at + i]] = tile * 32 + (int32_t)i;
         tile += nt;
     }
-    m.nbr.assign((size_t)tiles * nf * 32, 0);
+    // (a padding slot is its own neighbour: it starts at zero and stays there)
+    m.nbr.resize((size_t)tiles * nf * 32);
+    for (size_t i = 0; i < m.nbr.size(); ++i) m.nbr[i] = (int32_t)(i / (32 * nf) * 32 + i % 32);
     for (int64_t e = 0; e < op.nE; ++e)
         for (int f = 0; f < nf; ++f)
             m.nbr[((size_t)(m.slot[e] >> 5) * nf + f) * 32 + (m.slot[e] & 31)] = m.slot[op.nbr[e * nf + f]];
@@ -350,15 +352,20 @@ void finish_group(LaneTables &t, Writer &w, const std::vector<int32_t> &tail = {
     t.data.insert(t.data.end(), w.bytes.begin(), w.bytes.end());
 }
 
-// every element's geometry in its slot: [tile][element's values, faces' values][32]
+// every element's geometry in its slot: [tile][element's values, faces' values][32] (a
+// padding slot has that of its group's first element: the upwind wave divides by the faces'
+// normals)
 void lane_geometry(const HostOperators &op, const LaneMesh &m, std::vector<double> &geo) {
     const size_t eg = op.elem_geo.size() / op.nE, fg = op.face_geo.size() / op.nE, q = eg + fg;
-    geo.assign((size_t)m.n_slots * q, 0.0);
-    for (int64_t e = 0; e < op.nE; ++e) {
-        double *g = &geo[(size_t)(m.slot[e] >> 5) * q * 32 + (m.slot[e] & 31)];
+    geo.resize((size_t)m.n_slots * q);
+    auto put = [&](int64_t slot, int64_t e) {
+        double *g = &geo[(size_t)(slot >> 5) * q * 32 + (slot & 31)];
         for (size_t i = 0; i < eg; ++i) g[32 * i] = op.elem_geo[e * eg + i];
         for (size_t i = 0; i < fg; ++i) g[32 * (eg + i)] = op.face_geo[e * fg + i];
-    }
+    };
+    for (const LaneChunk &c : m.chunks)  // the last tile of a chunk may have padding
+        for (int i = 0; i < 32; ++i) put(32 * (int64_t)(c.tile0 + c.tiles - 1) + i, m.representative[c.group]);
+    for (int64_t e = 0; e < op.nE; ++e) put(m.slot[e], e);
 }
 
 }  // namespace

@@ -69,7 +69,7 @@ struct LaneChunk {
 struct LaneMesh {
     int64_t n_slots = 0;
     std::vector<int32_t> slot;         // [E]
-    std::vector<int32_t> nbr;          // [tile][nfl][32] the neighbours' slots (padding: 0)
+    std::vector<int32_t> nbr;          // [tile][nfl][32] the neighbours' slots (padding: its own)
     std::vector<LaneChunk> chunks;
     std::vector<int64_t> representative;  // [group] its first element
 };

@@ -2,7 +2,9 @@
 // arguments: cells along each axis, upper corner, triangular, order, physics (0, 1),
 // fp32, axis of the nodes to move (-1: none; dim: each node by its own amount along each
 // axis), by how much (relative to a cell; every other node plane).  Prints: "tensor <accepted>" or "groups <accepted> <number of groups>
-// <largest deviation of an element's geometry from its group's, relative to its own entry>".
+// <largest deviation of an element's geometry from its group's, relative to its own entry>
+// <padding slots> <those that are their own neighbour across every face> <smallest face
+// normal among the wave's plain tables' padding slots, 0 for other forms>".
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -84,7 +86,7 @@ int main(int argc, char **argv) {
     }
     LaneMesh lm;
     if (!lane_mesh(d, op, 1, !fp32, 64, 1 << 20, lm)) {
-        std::printf("groups 0 0 0\n");
+        std::printf("groups 0 0 0 0 0 0\n");
         return 0;
     }
     std::vector<int32_t> group(lm.n_slots / 32);
@@ -100,6 +102,27 @@ int main(int argc, char **argv) {
         for (int i = 0; i < eg; ++i) compare(op.elem_geo[e * eg + i], op.elem_geo[r * eg + i]);
         for (int i = 0; i < fg; ++i) compare(op.face_geo[e * fg + i], op.face_geo[r * fg + i]);
     }
-    std::printf("groups 1 %d %.3g\n", (int)lm.representative.size(), worst);
+    std::vector<uint8_t> used(lm.n_slots, 0);
+    for (int32_t s : lm.slot) used[s] = 1;
+    double least = 0.0;
+    LaneTables t;
+    if (physics && fp32 && lane_wave_tables(op, lm, false, 4, t)) least = 1e300;
+    int padding = 0, own = 0;
+    for (int64_t s = 0; s < lm.n_slots; ++s) {
+        if (used[s]) continue;
+        ++padding;
+        bool itself = true;
+        for (int f = 0; f < op.nfl; ++f) itself &= lm.nbr[((s >> 5) * op.nfl + f) * 32 + (s & 31)] == s;
+        own += itself;
+        for (int f = 0; f < op.nfl && !t.geometry.empty(); ++f) {
+            double q = 0.0;
+            for (int c = 0; c < dim; ++c) {
+                const double nu = t.geometry[((s >> 5) * (eg + fg) + eg + f * dim + c) * 32 + (s & 31)];
+                q += nu * nu;
+            }
+            least = std::min(least, std::sqrt(q));
+        }
+    }
+    std::printf("groups 1 %d %.3g %d %d %.3g\n", (int)lm.representative.size(), worst, padding, own, least);
     return 0;
 }

@@ -71,6 +71,17 @@ def test_cells_that_differ_keep_their_own(program, cells, upper, tri, wave, axis
 
 def test_graded_cells_are_refused(program):
     # every cell of its own size: more groups than tiles of them could fill
-    assert groups(program, [60, 64], [1.0, 1.0], True, 2, False, False, 2, 1e-4) == ["groups", "0", "0", "0"]
-    assert groups(program, [60, 64], [1.0, 1.0], True, 2, False, False, 2, 1e-11) == ["groups", "0", "0", "0"]
+    assert groups(program, [60, 64], [1.0, 1.0], True, 2, False, False, 2, 1e-4) == ["groups"] + ["0"] * 6
+    assert groups(program, [60, 64], [1.0, 1.0], True, 2, False, False, 2, 1e-11) == ["groups"] + ["0"] * 6
     assert groups(program, [33, 31], [1.0, 1.0], False, 2, False, False, 2, 1e-4) == ["tensor", "0"]
+
+
+@pytest.mark.parametrize("cells,tri", [([26, 22], True), ([9, 7], False), ([8, 6, 10], True)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_padding_stays_at_zero(program, cells, tri, fp32):
+    """A tile's padding slots are their own neighbours (they start at zero: their derivative
+    is zero), with a face normal the upwind wave can divide by."""
+    got = groups(program, cells, [1.0] * len(cells), tri, 2, True, fp32)
+    assert got[1] == "1" and int(got[4]) > 0 and got[5] == got[4], got
+    if fp32:
+        assert float(got[6]) > 0.0
