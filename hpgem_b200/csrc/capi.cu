@@ -129,6 +129,7 @@ __global__ void relayout(const T *src, T *dst, int nb, int64_t n, bool tiled, co
 
 int upload_tensor_geometry(hgg_handle *h);
 int alloc_tile_inputs(hgg_handle *h);
+int alloc_lin_inputs(hgg_handle *h);
 
 // moves every vector of a handle with a lane kernel between that kernel's layout and the
 // general kernels' (a change of the kernel variant; the padding elements stay zero)
@@ -136,6 +137,7 @@ int set_lane_layout(hgg_handle *h, bool lane) {
     int rc;
     if (!lane && h->op.tensor && (rc = upload_tensor_geometry(h))) return rc;
     if (!lane && h->group_tiles > 0 && (rc = alloc_tile_inputs(h))) return rc;
+    if (!lane && (rc = alloc_lin_inputs(h))) return rc;
     auto move = [&](auto *v) {
         using T = std::remove_pointer_t<decltype(v)>;
         T *tmp = reinterpret_cast<T *>(h->d_scratch);
@@ -374,6 +376,15 @@ int upload_tensor_geometry(hgg_handle *h) {
 int alloc_tile_inputs(hgg_handle *h) {
     for (int i = 0; i < 2; ++i)
         if (int rc = h->d_win[i] ? 0 : alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_win[i])) return rc;
+    return 0;
+}
+
+// ... and those of the stored-matrix tiles (where a chain tableau lets each stage form the
+// next one's input; not while a lane kernel runs the handle)
+int alloc_lin_inputs(hgg_handle *h) {
+    if (h->lin_tiles == 0 || h->umma_tiles > 0 || !chain_tableau(h)) return 0;
+    for (int i = 0; i < 2; ++i)
+        if (int rc = h->d_lin_win[i] ? 0 : alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_lin_win[i])) return rc;
     return 0;
 }
 
@@ -722,9 +733,7 @@ int attach_linear(hgg_handle *h, const LinearSystem &sys, int tiles_only) {
             (rc = upload(h, tmat, &h->d_lin_tile_mats)))
             return rc;
         h->lin_tiles = n_tiles;
-        if (u_tiles == 0)
-            for (int i = 0; i < 2; ++i)
-                if ((rc = alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_lin_win[i]))) return rc;
+        if (u_tiles == 0 && !h->lane && (rc = alloc_lin_inputs(h))) return rc;
     }
     if (u_tiles > 0) {
         // operand images of every distinct matrix: hi part then lo part, each NP x KP in the

@@ -91,7 +91,10 @@ thread_local std::string g_server_create_error = "no error";
 int64_t estimate_footprint(const hgg_problem_desc &d) {
     const int64_t N = d.n_elements * (int64_t)d.n_vars * d.n_basis;
     const int64_t kbytes = d.precision == HGG_PRECISION_FP32 ? 4 : 8;
-    const int64_t ahead = d.physics == HGG_PHYSICS_ADVECTION ? 0 : 2 * 8;  // wave: stage inputs formed ahead
+    // stage inputs formed ahead: the wave's, and those of folded triangles in the FP32 form
+    // (the other folded ones run on the lane kernels, which form none)
+    const bool folded = d.shape == HGG_SHAPE_TRIANGLE && d.n_basis >= 21 && d.precision == HGG_PRECISION_FP32;
+    const int64_t ahead = d.physics != HGG_PHYSICS_ADVECTION || folded ? 2 * 8 : 0;
     return (3 * 8 + ahead + d.n_stages * kbytes) * (N + 64 * 64) + d.n_elements * 640 + (8 << 20);
 }
 
