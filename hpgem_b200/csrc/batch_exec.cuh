@@ -362,7 +362,7 @@ bool same_class(const BatchClass &c, const hgg_handle *h) {
     return c.kind == batch_kind(h) && c.shape == h->op.shape && c.order == h->op.order && c.dim == h->op.dim &&
            c.physics == h->op.physics && c.mixed == h->mixed && c.S == h->S && c.rk_a == h->rk_a &&
            c.rk_b == h->rk_b &&
-           (c.kind != KIND_LANE || c.rep.nB == h->op.nB) && (c.kind != KIND_LINEAR || c.rows == h->lin_R) &&
+           (c.kind != KIND_LANE || c.rep.nB == h->op.nB) && (c.kind != KIND_LINEAR || (c.rows == h->lin_R && c.chain == lin_forms_input(h, true))) &&
            (c.kind != KIND_UMMA || (c.precision == h->precision && c.rows == h->lin_R && c.lslots == h->lin_slots));
 }
 

@@ -39,7 +39,10 @@ int fail(hgg_handle *h, int code, const std::string &msg) {
 int alloc(hgg_handle *h, size_t bytes, void **dst) {
     void *p = nullptr;
     cudaError_t e = cudaMallocAsync(&p, bytes, h->stream);
-    if (e != cudaSuccess) return fail(h, HGG_ERR_NOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // (not left for the next launch's check: the caller may go on without)
+        return fail(h, HGG_ERR_NOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+    }
     h->bufs.push_back({p, bytes});
     *dst = p;
     return 0;
@@ -128,16 +131,16 @@ __global__ void relayout(const T *src, T *dst, int nb, int64_t n, bool tiled, co
 }
 
 int upload_tensor_geometry(hgg_handle *h);
-int alloc_tile_inputs(hgg_handle *h);
-int alloc_lin_inputs(hgg_handle *h);
+void alloc_tile_inputs(hgg_handle *h);
+void alloc_lin_inputs(hgg_handle *h);
 
 // moves every vector of a handle with a lane kernel between that kernel's layout and the
 // general kernels' (a change of the kernel variant; the padding elements stay zero)
 int set_lane_layout(hgg_handle *h, bool lane) {
     int rc;
     if (!lane && h->op.tensor && (rc = upload_tensor_geometry(h))) return rc;
-    if (!lane && h->group_tiles > 0 && (rc = alloc_tile_inputs(h))) return rc;
-    if (!lane && (rc = alloc_lin_inputs(h))) return rc;
+    if (!lane) alloc_tile_inputs(h);
+    if (!lane) alloc_lin_inputs(h);
     auto move = [&](auto *v) {
         using T = std::remove_pointer_t<decltype(v)>;
         T *tmp = reinterpret_cast<T *>(h->d_scratch);
@@ -372,20 +375,22 @@ int upload_tensor_geometry(hgg_handle *h) {
     return 0;
 }
 
-// stage inputs the tile kernel of the wave forms ahead
-int alloc_tile_inputs(hgg_handle *h) {
-    for (int i = 0; i < 2; ++i)
-        if (int rc = h->d_win[i] ? 0 : alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_win[i])) return rc;
-    return 0;
+// Stage inputs formed ahead, two vectors: where there is no memory for them the stages read
+// several vectors instead.
+void alloc_inputs(hgg_handle *h, double *(&win)[2]) {
+    double *both = nullptr;
+    if (win[0] || alloc(h, 2 * sizeof(double) * h->N_alloc, (void **)&both)) return;
+    win[0] = both;
+    win[1] = both + h->N_alloc;
 }
-
-// ... and those of the stored-matrix tiles (where a chain tableau lets each stage form the
-// next one's input; not while a lane kernel runs the handle)
-int alloc_lin_inputs(hgg_handle *h) {
-    if (h->lin_tiles == 0 || h->umma_tiles > 0 || !chain_tableau(h)) return 0;
-    for (int i = 0; i < 2; ++i)
-        if (int rc = h->d_lin_win[i] ? 0 : alloc(h, sizeof(double) * h->N_alloc, (void **)&h->d_lin_win[i])) return rc;
-    return 0;
+// those of the wave's tile kernel
+void alloc_tile_inputs(hgg_handle *h) {
+    if (h->group_tiles > 0) alloc_inputs(h, h->d_win);
+}
+// ... and of the stored-matrix tiles (where a chain tableau lets each stage form the next
+// one's input; not while a lane kernel runs the handle)
+void alloc_lin_inputs(hgg_handle *h) {
+    if (h->lin_tiles > 0 && h->umma_tiles == 0 && chain_tableau(h)) alloc_inputs(h, h->d_lin_win);
 }
 
 // Lane kernel of simplices and of the wave: the mesh's groups, their tables (host).
@@ -444,7 +449,8 @@ int upload_lane(hgg_handle *h, const LaneMesh &m, const LaneTables &t) {
 
 // linear: the handle will run the stored-matrix kernel (attach_linear), so the
 // vectors stay in hpGEM order and the matrix-free operators are not uploaded
-int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = false) {
+// lanes: the lane kernels may be taken
+int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = false, bool lanes = true) {
     try {
         h->op = build_operators(*desc, !linear);
     } catch (const std::exception &ex) {
@@ -471,10 +477,10 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
         vectors = std::max(vectors, n);
     }
     const bool one_shot = h->mixed && vectors > 2 && op.nB >= 16 && op.nE < 185 * 32;
-    h->lane_ok = h->lane = !h->slice_ok && !one_shot && tensor_lane_setup(*desc, op, h->mixed, h->tlane, lane_nbr);
+    h->lane_ok = h->lane = lanes && !h->slice_ok && !one_shot && tensor_lane_setup(*desc, op, h->mixed, h->tlane, lane_nbr);
     LaneMesh lmesh;
     LaneTables ltab;
-    if (!op.tensor && !linear && desc->precision != HGG_PRECISION_BF16X3) lane_setup(h, *desc, lmesh, ltab);
+    if (lanes && !op.tensor && !linear && desc->precision != HGG_PRECISION_BF16X3) lane_setup(h, *desc, lmesh, ltab);
     h->tiled = h->slice_ok || h->lane;
     if (h->slice_ok) h->tile_elems = SliceShape::TE;
     if (h->mixed && !mixed_supported(h))
@@ -614,7 +620,7 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
             if (n_tiles * TE <= 2 * op.nE) {
                 if ((rc = upload(h, tiles, &h->d_group_tiles))) return rc;
                 h->group_tiles = n_tiles;
-                if (!h->lane_ok && (rc = alloc_tile_inputs(h))) return rc;
+                if (!h->lane_ok) alloc_tile_inputs(h);
             }
             // (before any change of the variant: the kernel the lane kernel stands in for)
             h->lgeo.neighbour_fp64 = group_wave_wanted(h);
@@ -733,7 +739,7 @@ int attach_linear(hgg_handle *h, const LinearSystem &sys, int tiles_only) {
             (rc = upload(h, tmat, &h->d_lin_tile_mats)))
             return rc;
         h->lin_tiles = n_tiles;
-        if (u_tiles == 0 && !h->lane && (rc = alloc_lin_inputs(h))) return rc;
+        if (u_tiles == 0 && !h->lane) alloc_lin_inputs(h);
     }
     if (u_tiles > 0) {
         // operand images of every distinct matrix: hi part then lo part, each NP x KP in the
@@ -818,16 +824,22 @@ extern "C" {
 int hgg_create(const hgg_problem_desc *desc, hgg_handle **out) {
     if (!desc || !out) return fail(nullptr, HGG_ERR_INVALID, "null argument");
     *out = nullptr;
-    hgg_handle *h = new (std::nothrow) hgg_handle();
-    if (!h) return fail(nullptr, HGG_ERR_NOMEM, "host allocation failed");
-    int rc = create_from_desc(desc, h);
-    if (rc) {
+    // (the lane kernels' vectors have padding and want one more for their conversion: a
+    // problem that fits the device only without them gets the general kernels)
+    for (bool lanes : {true, false}) {
+        hgg_handle *h = new (std::nothrow) hgg_handle();
+        if (!h) return fail(nullptr, HGG_ERR_NOMEM, "host allocation failed");
+        const int rc = create_from_desc(desc, h, false, lanes);
+        if (!rc) {
+            *out = h;
+            return 0;
+        }
+        const bool again = rc == HGG_ERR_NOMEM && h->lane_ok;
         g_create_error = h->err;
         destroy_handle(h);
-        return rc;
+        if (!again) return rc;
     }
-    *out = h;
-    return 0;
+    return HGG_ERR_NOMEM;
 }
 
 int hgg_destroy(hgg_handle *h) {

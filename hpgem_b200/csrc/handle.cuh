@@ -147,23 +147,21 @@ int fail(hgg_handle *h, int code, const std::string &msg);
 // work of other streams, so a solve that finishes inside a batch or a server is freed
 // while the other members keep stepping.
 
+int alloc(hgg_handle *h, size_t bytes, void **dst);
 // device copy of a host vector, owned by the handle
 template <typename T>
 int upload(hgg_handle *h, const std::vector<T> &v, T **dst) {
     *dst = nullptr;
     if (v.empty()) return 0;
+    const size_t bytes = v.size() * sizeof(T);
     void *p = nullptr;
-    size_t bytes = v.size() * sizeof(T);
-    cudaError_t e = cudaMallocAsync(&p, bytes, h->stream);
-    if (e != cudaSuccess) return fail(h, HGG_ERR_NOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-    h->bufs.push_back({p, bytes});
-    e = cudaMemcpyAsync(p, v.data(), bytes, cudaMemcpyHostToDevice, h->stream);
+    if (int rc = alloc(h, bytes, &p)) return rc;
+    cudaError_t e = cudaMemcpyAsync(p, v.data(), bytes, cudaMemcpyHostToDevice, h->stream);
     if (e != cudaSuccess) return fail(h, HGG_ERR_CUDA, std::string("cudaMemcpyAsync: ") + cudaGetErrorString(e));
     *dst = (T *)p;
     return 0;
 }
 
-int alloc(hgg_handle *h, size_t bytes, void **dst);
 // coefficients per element (all variables)
 inline int coefficients(const hgg_handle *h) { return h->op.V * h->op.nB; }
 // the wave runs the grouped tile kernel (alone and in a batch): kernel variant 2, or
