@@ -303,6 +303,7 @@ struct hgg_batch {
     cudaEvent_t fork = nullptr;
     std::vector<hgg_handle *> handles;  // by slot, nullptr when free
     std::vector<std::shared_ptr<int>> membership;  // by slot: the handle's count of batches
+    int64_t sparse_tiles = 0;           // lane tiles that are mostly padding, of all members
     std::vector<double> dt;
     std::vector<int> base;               // the handle's current buffer when it was added
     std::vector<int> cls;                // class index of each slot
@@ -1037,6 +1038,7 @@ int remove_member(hgg_batch *b, int slot, int parity) {
     c.slots.erase(std::find(c.slots.begin(), c.slots.end(), slot));
     c.table_dirty = true;
     b->handles[slot] = nullptr;
+    if (h->lane && h->lane_sparse) b->sparse_tiles -= h->lgeo.n_slots / 32;
     --*b->membership[slot];
     b->membership[slot].reset();
     b->cls[slot] = -1;
@@ -1118,6 +1120,14 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
         return bfail(b, HGG_ERR_UNSUPPORTED, "dense kernel: more than 256 coefficients per element");
     // the handle's own work must be finished before the batch uses its buffers
     HGG_BCUDA(b, cudaStreamSynchronize(h->stream));
+    // Lane tiles that are mostly padding pay while all of them run at once, as alone, not in
+    // a batch of many: 64 meshes of 128 triangles that all differ took, advection at p = 1
+    // and 3, 93 and 237 us per step on the lane kernels, 35 and 38 on the general ones; 16 of
+    // 32 such triangles 19 and 23 against 29 and 33.  Members beyond two such tiles per SM
+    // take the general kernels.
+    const int64_t tiles = h->lane && h->lane_sparse ? h->lgeo.n_slots / 32 : 0;
+    const bool general = tiles > 0 && b->sparse_tiles + tiles > 2 * (int64_t)b->num_sms;
+    if (settle_layout(h, general)) return bfail(b, HGG_ERR_CUDA, hgg_last_error(h));
     int ci = -1;
     for (size_t i = 0; i < b->classes.size(); ++i)
         if (same_class(b->classes[i], h)) ci = (int)i;
@@ -1172,6 +1182,7 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
     b->classes[ci].table_dirty = true;
     b->item_cache[free_slot].clear();  // formed at the next table upload
     b->handles[free_slot] = h;
+    if (!general) b->sparse_tiles += tiles;
     b->membership[free_slot] = h->memberships;
     ++*h->memberships;
     b->dt[free_slot] = dt;

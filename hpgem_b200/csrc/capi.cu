@@ -164,8 +164,8 @@ int set_lane_layout(hgg_handle *h, bool lane) {
     return 0;
 }
 
-int settle_layout(hgg_handle *h) {
-    const bool lane = h->lane_ok && h->variant == 0;
+int settle_layout(hgg_handle *h, bool general) {
+    const bool lane = h->lane_ok && h->variant == 0 && !general;
     if (lane == h->lane || *h->memberships > 0) return 0;
     release_graphs(h);
     return set_lane_layout(h, lane);
@@ -417,6 +417,7 @@ void lane_setup(hgg_handle *h, const hgg_problem_desc &desc, LaneMesh &m, LaneTa
                 : lane_advection_tables(op, m, folded, elem_bytes, t))) return;
     if (t.group_bytes > 96 * 1024) return;
     h->lane_ok = h->lane = h->tensor_layout = true;
+    h->lane_sparse = m.sparse;
 }
 
 int upload_lane(hgg_handle *h, const LaneMesh &m, const LaneTables &t) {

@@ -84,6 +84,9 @@ struct hgg_handle {
     hgg::LaneGeom lgeo{};                  // simplices and the wave
     double *d_lane_win[2] = {nullptr, nullptr};  // ... the wave: stage inputs formed ahead (contraction type)
     int lane_tiles = 1;                    // ... tiles of a chunk at most
+    // ... mostly padding: faster than the general kernels only while all tiles run at once
+    // (see hgg_batch_add)
+    bool lane_sparse = false;
     std::vector<int32_t> slot;            // place of each element in the lane layout (empty: its own number)
     int32_t *d_slot = nullptr;            // slot on the device while the lane layout is in use, else null
     int32_t *d_slot_lane = nullptr;
@@ -168,8 +171,9 @@ inline int coefficients(const hgg_handle *h) { return h->op.V * h->op.nB; }
 // the automatic choice where it measured faster than the per-row kernel
 bool group_wave_wanted(const hgg_handle *h);
 void release_graphs(hgg_handle *h);
-// the vectors into the layout of the kernel variant, unless a batch steps them
-int settle_layout(hgg_handle *h);
+// the vectors into the layout of the kernel variant, or (general) of the general kernels,
+// unless a batch steps them
+int settle_layout(hgg_handle *h, bool general = false);
 // the current solution in hpGEM order with no kernel on the device: one copy of the
 // device vector into `staging` (pinned, h->N_alloc doubles), the layout change on the host
 int solution_to_host(hgg_handle *h, double *staging, double *out);

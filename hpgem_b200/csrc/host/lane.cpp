@@ -268,8 +268,11 @@ bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_
     const int64_t pad = tiles * 32 - op.nE;
     // padded slots cost idle lanes and memory in every vector: at most twice as many as
     // elements (a full tile's element costs a third of the general kernels') unless all
-    // tiles run at once, and within spare_bytes per element and 4 MB
-    if (pad > 2 * op.nE && tiles > 2 * 148) return false;
+    // tiles run at once, and within spare_bytes per element and 4 MB.  (A tile of one element
+    // is then still the faster: 128 triangles that all differ, advection at p = 3 12.1 us per
+    // RK4 step against 24.9, the wave at p = 1 12.7 against 32.8.)
+    m.sparse = pad > 2 * op.nE;
+    if (m.sparse && tiles > 2 * 148) return false;
     if ((double)pad * R * coefficient_bytes > (double)spare_bytes * (double)op.nE + 4e6) return false;
     if (tiles > INT32_MAX / 32) return false;
     m.n_slots = tiles * 32;

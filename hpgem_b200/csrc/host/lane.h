@@ -68,6 +68,7 @@ struct LaneChunk {
 };
 struct LaneMesh {
     int64_t n_slots = 0;
+    bool sparse = false;               // more than twice as many padding slots as elements
     std::vector<int32_t> slot;         // [E]
     std::vector<int32_t> nbr;          // [tile][nfl][32] the neighbours' slots (padding: its own)
     std::vector<LaneChunk> chunks;

@@ -16,9 +16,11 @@ def kernel_class(solver):
     return kind
 
 
-def write_mesh_file(path, axes, triangles=False):
+def write_mesh_file(path, axes, triangles=False, jiggle=0.0):
     """A periodic "mesh 2" file: nodes at the products of `axes` (each from the lower to the
-    upper corner, both included), quadrilaterals, hexahedra or two triangles per cell."""
+    upper corner, both included), each then moved by up to `jiggle` cells of its own;
+    quadrilaterals, hexahedra or two triangles per cell."""
+    rng = np.random.default_rng(7)
     dim, cells = len(axes), [len(a) - 1 for a in axes]
     number = {}
     lines = []
@@ -26,10 +28,11 @@ def write_mesh_file(path, axes, triangles=False):
         idx = idx[::-1]
         number[idx] = len(number)
         wraps = [c for c in range(dim) if idx[c] == 0]
+        off = [jiggle * rng.uniform(-1.0, 1.0) * (axes[c][-1] - axes[c][0]) / cells[c] for c in range(dim)]
         copies = []
         for sub in range(1 << len(wraps)):
             far = [c for b, c in enumerate(wraps) if sub >> b & 1]
-            copies.append([axes[c][cells[c] if c in far else idx[c]] for c in range(dim)])
+            copies.append([axes[c][cells[c] if c in far else idx[c]] + off[c] for c in range(dim)])
         lines += ["1 0", "%d %s" % (len(copies), " ".join(float(v).hex() for x in copies for v in x))]
     corners = [[0, 1, 2], [1, 3, 2]] if triangles else [list(range(1 << dim))]
     elements = []

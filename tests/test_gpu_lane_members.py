@@ -7,7 +7,7 @@ import pytest
 
 import hpgem_b200
 
-from lane_helpers import kernel_class
+from lane_helpers import kernel_class, write_mesh_file
 
 pytestmark = pytest.mark.gpu
 
@@ -85,3 +85,43 @@ def test_source_set_on_a_stored_matrix_member():
     solvers[1].handle.step(0.0, 1e-4, 3)
     want = solvers[1].handle.get_state(0)
     assert np.abs(solvers[0].handle.get_state(0) - want).max() < 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("cells,order,physics,alone", [([8, 8], 3, "advection", 2), ([6, 6], 1, "wave", 4), ([4, 4], 4, "advection", 9)])
+def test_batches_step_many_sparse_tiles_with_the_general_kernels(tmp_path, cells, order, physics, alone):
+    """A small mesh whose triangles all differ has a tile for each of them: the lane kernel is
+    the faster for as many such meshes as run at once (two tiles per SM: `alone` of these),
+    the others of a batch take the general kernels.  Their vectors go back when they leave."""
+    path = write_mesh_file(tmp_path / "mesh.hpgem", [np.linspace(0.0, 1.0, n + 1) for n in cells], True, 0.1)
+    solvers = []
+    for i in range(alone + 3):
+        if physics == "advection":
+            s = hpgem_b200.Advection(2, order, [0.7, -0.4], tableau="RK4_4").readMeshFile(path)
+        else:
+            s = hpgem_b200.AcousticWave(2, order, c_inv=0.8, tableau="RK4_4", flux="upwind").readMeshFile(path)
+        s.handle.set_state(0, np.random.default_rng(6).standard_normal(s.handle.vector_length))
+        solvers.append(s)
+    ref = solvers.pop()
+    dt = 0.01 / max(cells) / (2 * order + 1) ** 2
+    batch = hpgem_b200.Batch(len(solvers) + 1)
+    slots = [batch.add(s, dt, 5) for s in solvers]
+    members = {c["kind"]: c["members"] for c in batch.class_info()}
+    assert members.pop("lane tables") == alone and list(members.values()) == [2]
+    batch.step(5)
+    batch.synchronize()
+    halves = [s.handle.get_state(0) for s in solvers]
+    for slot in slots:
+        batch.remove(slot)
+    again = batch.add(solvers[-1], dt, 4)  # there is room among the tiles again
+    assert [c["kind"] for c in batch.class_info()] == ["lane tables"]
+    assert np.array_equal(solvers[-1].handle.get_state(0), halves[-1])
+    batch.step(4)
+    batch.synchronize()
+    batch.remove(again)
+    batch.close()
+    ref.handle.step(0.0, dt, 9)
+    want = ref.handle.get_state(0)
+    for s in solvers[:-1]:
+        s.handle.step(0.0, dt, 4)
+    for s in solvers:
+        assert np.abs(s.handle.get_state(0) - want).max() < 1e-12 * np.abs(want).max()
