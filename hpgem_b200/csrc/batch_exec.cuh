@@ -1183,6 +1183,7 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
     b->item_cache[free_slot].clear();  // formed at the next table upload
     b->handles[free_slot] = h;
     if (!general) b->sparse_tiles += tiles;
+    if (!h->memberships) h->memberships = std::make_shared<int>(0);
     b->membership[free_slot] = h->memberships;
     ++*h->memberships;
     b->dt[free_slot] = dt;

@@ -166,7 +166,7 @@ int set_lane_layout(hgg_handle *h, bool lane) {
 
 int settle_layout(hgg_handle *h, bool general) {
     const bool lane = h->lane_ok && h->variant == 0 && !general;
-    if (lane == h->lane || *h->memberships > 0) return 0;
+    if (lane == h->lane || (h->memberships && *h->memberships > 0)) return 0;
     release_graphs(h);
     return set_lane_layout(h, lane);
 }
@@ -820,6 +820,20 @@ int capture_steps(hgg_handle *h, int from, int steps, double dt, cudaGraphExec_t
 }
 }  // namespace
 
+namespace {
+// f's code, or that of the exception it ended with: none crosses the C boundary
+template <typename F>
+int returning(hgg_handle *h, F &&f) {
+    try {
+        return f();
+    } catch (const std::bad_alloc &) {
+        return fail(h, HGG_ERR_NOMEM, "host allocation failed");
+    } catch (const std::exception &ex) {
+        return fail(h, HGG_ERR_INVALID, ex.what());
+    }
+}
+}  // namespace
+
 extern "C" {
 
 int hgg_create(const hgg_problem_desc *desc, hgg_handle **out) {
@@ -830,7 +844,7 @@ int hgg_create(const hgg_problem_desc *desc, hgg_handle **out) {
     for (bool lanes : {true, false}) {
         hgg_handle *h = new (std::nothrow) hgg_handle();
         if (!h) return fail(nullptr, HGG_ERR_NOMEM, "host allocation failed");
-        const int rc = create_from_desc(desc, h, false, lanes);
+        const int rc = returning(h, [&] { return create_from_desc(desc, h, false, lanes); });
         if (!rc) {
             *out = h;
             return 0;
@@ -1007,7 +1021,7 @@ int hgg_set_kernel_variant(hgg_handle *h, int32_t variant) {
     const int was = h->variant;
     if (variant != was) release_graphs(h);
     h->variant = variant;
-    const int rc = settle_layout(h);
+    const int rc = returning(h, [&] { return settle_layout(h); });
     if (rc) h->variant = was;
     return rc;
 }

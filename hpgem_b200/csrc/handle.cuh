@@ -78,7 +78,7 @@ struct hgg_handle {
     // batches that have the handle as a member: their tables hold its vectors' layout, so a
     // change of the variant moves them when the last has let go (shared with the batch,
     // which may outlive the handle)
-    std::shared_ptr<int> memberships = std::make_shared<int>(0);
+    std::shared_ptr<int> memberships;  // (null: never in one)
     bool overlap = true;                  // chained launches start early (hgg_test_set_overlap)
     hgg::TensorLaneGeom tlane{};          // sum-factorised handles
     hgg::LaneGeom lgeo{};                  // simplices and the wave
