@@ -309,6 +309,16 @@ int set_tableau(hgg_handle *h, int32_t n_stages, const double *a, const double *
     return 0;
 }
 
+// of the current device (without one, a B200's: creation fails later, with its own code)
+int device_sms() {
+    int device = 0, n = 0;
+    if (cudaGetDevice(&device) == cudaSuccess &&
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0)
+        return n;
+    cudaGetLastError();
+    return 148;
+}
+
 // device, stream, solution and stage vectors (N_alloc doubles each), status word
 int init_device_vectors(hgg_handle *h) {
     int ndev = 0;
@@ -407,12 +417,12 @@ void lane_setup(hgg_handle *h, const hgg_problem_desc &desc, LaneMesh &m, LaneTa
     // a block takes several tiles of a group once every SM has two such blocks: the group's
     // table is then read from L2 once for all of them
     const int most = std::max(1, 4 / lane_warps(op.nB, wave ? lane_wave_rows(folded) : kLaneAdvRows));
-    h->lane_tiles = op.nE / 32 >= 2 * (int64_t)most * 148 ? most : 1;
+    h->lane_tiles = op.nE / 32 >= 2 * (int64_t)most * h->num_sms ? most : 1;
     const int bytes = 24 + (wave ? 2 * elem_bytes : 0) + h->S * (h->mixed ? 4 : 8);
     // a server's estimate of a handle's footprint leaves 320 bytes per element and 4 MB, and
     // the FP32 wave's stage inputs are half of what it counts
     const int spare = 320 + (wave && elem_bytes == 4 ? 8 * op.V * op.nB : 0);
-    if (!lane_mesh(desc, op, h->lane_tiles, folded, bytes, spare, m)) return;
+    if (!lane_mesh(desc, op, h->num_sms, h->lane_tiles, folded, bytes, spare, m)) return;
     if (!(wave ? lane_wave_tables(op, m, folded, elem_bytes, t)
                 : lane_advection_tables(op, m, folded, elem_bytes, t))) return;
     if (t.group_bytes > 96 * 1024) return;
@@ -469,15 +479,16 @@ int create_from_desc(const hgg_problem_desc *desc, hgg_handle *h, bool linear = 
     std::vector<int32_t> lane_nbr;
     // In the FP32 form a stage that reads many vectors (Dormand-Prince) is a long chain of
     // loads for a thread with a whole element of 16 or more functions: below a warp or so
-    // per SM the one-shot kernel's thread per coefficient is faster (per step 32 x 45 p = 5
-    // 33 against 44 us, 60^2 p = 4 33 against 43; 100 x 90 p = 5 64 against 53)
+    // (five quarters) per SM the one-shot kernel's thread per coefficient is faster (per step
+    // 32 x 45 p = 5 33 against 44 us, 60^2 p = 4 33 against 43; 100 x 90 p = 5 64 against 53)
     int vectors = 0;
     for (int i = 0; i < h->S; ++i) {
         int n = 0;
         for (int j = 0; j < i; ++j) n += h->rk_a[i * h->S + j] != 0.0;
         vectors = std::max(vectors, n);
     }
-    const bool one_shot = h->mixed && vectors > 2 && op.nB >= 16 && op.nE < 185 * 32;
+    h->num_sms = device_sms();
+    const bool one_shot = h->mixed && vectors > 2 && op.nB >= 16 && op.nE < 40 * (int64_t)h->num_sms;
     h->lane_ok = h->lane = lanes && !h->slice_ok && !one_shot && tensor_lane_setup(*desc, op, h->mixed, h->tlane, lane_nbr);
     LaneMesh lmesh;
     LaneTables ltab;

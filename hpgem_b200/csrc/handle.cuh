@@ -179,12 +179,12 @@ int settle_layout(hgg_handle *h, bool general = false);
 int solution_to_host(hgg_handle *h, double *staging, double *out);
 
 // Launch of a stage kernel that calls chain_next and chain_wait: with `overlap` its start
-// overlaps the previous kernel's end on the same stream (anything else before it is waited for in
-// full), which takes most of the gap between two stages out.  Per RK4 step: 32^2
-// quadrilaterals at p = 2 12.7 -> 9.1 us, triangles 192 x 160 at p = 3 22.6 -> 17.9, the
-// FP32 wave on 14 x 18 x 12 x 5 tetrahedra at p = 3 160 -> 154.  (Letting the next stage
-// start at a kernel's beginning instead of before its outputs spreads its blocks unevenly
-// over the SMs: the triangles took 23.7.)
+// overlaps the previous kernel's end on the same stream (anything else before it is waited
+// for in full), which takes part of the gap between two stages out.  Per RK4 step in graphs
+// of eight steps: 32^2 quadrilaterals at p = 2 10.3 -> 9.5 us, triangles 192 x 160 at p = 3
+// 20.4 -> 17.9, the FP32 wave on 14 x 18 x 12 x 5 tetrahedra at p = 3 130 -> 127.  (Letting
+// the next stage start at a lane kernel's beginning instead of before its outputs spreads
+// its blocks unevenly over the SMs: the triangles took 23.7.)
 template <typename... K, typename... A>
 void launch_chained(bool overlap, void (*kern)(K...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
                     A &&...args) {

@@ -180,7 +180,7 @@ bool tensor_lane_setup(const hgg_problem_desc &desc, const HostOperators &op, bo
 
 // ---- simplices and the wave -------------------------------------------------------
 
-bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_tiles_max, bool folded,
+bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int num_sms, int chunk_tiles_max, bool folded,
                int coefficient_bytes, int spare_bytes, LaneMesh &m) {
     const int nf = op.nfl, d = op.dim, R = op.V * op.nB;
     const bool wave = op.physics != 0;
@@ -216,7 +216,7 @@ bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_
         dst[n] = (uint64_t)(int64_t)e;
         return true;
     };
-    const size_t most = (size_t)op.nE / 10 + 296;  // more groups than this take too much padding
+    const size_t most = (size_t)op.nE / 10 + 2 * num_sms;  // more groups than this take too much padding
     std::optional<GeometryRounding> rounding;
     if (folded) rounding.emplace(desc, op);
     std::vector<double> bounds;  // [group][eg + nf fg]
@@ -272,7 +272,7 @@ bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_
     // is then still the faster: 128 triangles that all differ, advection at p = 3 12.1 us per
     // RK4 step against 24.9, the wave at p = 1 12.7 against 32.8.)
     m.sparse = pad > 2 * op.nE;
-    if (m.sparse && tiles > 2 * 148) return false;
+    if (m.sparse && tiles > 2 * num_sms) return false;
     if ((double)pad * R * coefficient_bytes > (double)spare_bytes * (double)op.nE + 4e6) return false;
     if (tiles > INT32_MAX / 32) return false;
     m.n_slots = tiles * 32;

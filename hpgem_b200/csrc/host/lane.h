@@ -113,7 +113,7 @@ struct LaneTables {
 // (unstructured meshes, very small ones).
 // coefficient_bytes: of all vectors of the handle, per coefficient; spare_bytes: what the
 // padding may take per element (and 4 MB).
-bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int chunk_tiles_max, bool folded,
+bool lane_mesh(const hgg_problem_desc &desc, const HostOperators &op, int num_sms, int chunk_tiles_max, bool folded,
                int coefficient_bytes, int spare_bytes, LaneMesh &m);
 // Tables of the groups: `folded` as described in lane_stage.cuh, or plain with entries of
 // elem_bytes; false when the operators

@@ -23,10 +23,10 @@
 //     operations in their order (plain tables, every element's own geometry), so their
 //     results are the general kernels' bit for bit.
 // Measured, us per RK4 step, the general kernel against this one: the upwind wave on
-// 32^3 x 5 tetrahedra at p = 2 972 -> 266 (FP64), 835 -> 399 (FP32), 14 x 18 x 12 x 5 at
-// p = 3 296 -> 109 and 241 -> 160, 128^2 x 2 triangles at p = 4 241 -> 68 and 190 -> 103;
-// advection on 192 x 160 x 2 triangles at p = 3 122 -> 23 and 81 -> 35, on 16^3 x 5
-// tetrahedra at p = 3 162 -> 39 and 118 -> 61.
+// 32^3 x 5 tetrahedra at p = 2 971 -> 260 (FP64), 831 -> 376 (FP32), the wave on
+// 14 x 18 x 12 x 5 at p = 3 297 -> 97 and 239 -> 127, on 128^2 x 2 triangles at p = 4
+// 217 -> 62 and 174 -> 86; advection on 192 x 160 x 2 triangles at p = 3 120 -> 18 and
+// 78 -> 23, on 16^3 x 5 tetrahedra at p = 3 160 -> 26 and 116 -> 48.
 #pragma once
 
 #include <cstdint>

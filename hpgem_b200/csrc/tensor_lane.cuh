@@ -16,13 +16,11 @@
 //     the outflow face's lift sigma l (x) trace fold on the host into one 1D matrix
 //     per axis, E_c = ahat_c D1 - sigma l_side (x) e_side, which the stage reads from
 //     the kernel's parameters (the FP32 form keeps the general kernel's order of
-//     operations instead, so its results do not change by FP32 roundings); per axis one inflow face remains, whose neighbour
-//     index is all the geometry an element reads (4 bytes per axis; the general
-//     kernels read 112 bytes per element in 3D).
-// Measured (whole solves of 100 RK4 steps with their host copies, against the pipelined
-// kernel): 32^2 quadrilaterals at p = 2 23.0 -> 12.7 us per step, 150 x 210 at p = 4
-// 72.6 -> 23.3 us; 96 small problems in a batch (FP32 form, half of them on
-// quadrilaterals) 71.3 -> 56.0 ms per 50 steps.
+//     operations instead, so its results do not change by FP32 roundings); per axis one
+//     inflow face remains, whose neighbour index is all the geometry an element reads
+//     (4 bytes per axis; the general kernels read 112 bytes per element in 3D).
+// Measured, us per RK4 step, the one-shot and the pipelined kernel against this one: 32^2
+// quadrilaterals at p = 2 17.7 and 20.3 -> 9.5, 150 x 210 at p = 4 56.0 and 65.8 -> 17.8.
 #pragma once
 
 #include <cstdint>

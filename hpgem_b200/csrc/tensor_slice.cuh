@@ -274,8 +274,8 @@ __device__ __forceinline__ void tensor_slice_body(const StageIOT<KT> &io, const 
 }
 
 // One block per 32-element tile of one problem, chained to the previous stage (chain_next,
-// chain_wait): the last wave's idle SMs start the next stage (64^3: 513 -> 495 us per RK4
-// step, FP32 425 -> 407; 10^3: 31.0 -> 27.6).  Five blocks per SM (102
+// chain_wait): the last wave's idle SMs start the next stage (64^3: 513 -> 492 us per RK4
+// step, FP32 393 -> 368; 10^3: 29.2 -> 25.4).  Five blocks per SM (102
 // registers, a little spilling) for the stages without the final update: the
 // extra resident warps measured 1.6 % faster per RK4 step than four blocks;
 // the final stage, which holds 16 more values per thread, keeps four.

@@ -85,7 +85,7 @@ int main(int argc, char **argv) {
         return 0;
     }
     LaneMesh lm;
-    if (!lane_mesh(d, op, 1, !fp32, 64, 1 << 20, lm)) {
+    if (!lane_mesh(d, op, 148, 1, !fp32, 64, 1 << 20, lm)) {
         std::printf("groups 0 0 0 0 0 0\n");
         return 0;
     }
