@@ -1125,8 +1125,8 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
     // and 3, 93 and 237 us per step on the lane kernels, 35 and 38 on the general ones; 16 of
     // 32 such triangles 19 and 23 against 29 and 33.  Members beyond two such tiles per SM
     // take the general kernels.
-    const int64_t tiles = h->lane && h->lane_sparse ? h->lgeo.n_slots / 32 : 0;
-    const bool general = tiles > 0 && b->sparse_tiles + tiles > 2 * (int64_t)b->num_sms;
+    const bool general =
+        h->lane_sparse && b->sparse_tiles + h->lgeo.n_slots / 32 > 2 * (int64_t)b->num_sms;
     if (settle_layout(h, general)) return bfail(b, HGG_ERR_CUDA, hgg_last_error(h));
     int ci = -1;
     for (size_t i = 0; i < b->classes.size(); ++i)
@@ -1182,7 +1182,8 @@ int hgg_batch_add(hgg_batch *b, hgg_handle *h, double dt, int32_t nsteps, int32_
     b->classes[ci].table_dirty = true;
     b->item_cache[free_slot].clear();  // formed at the next table upload
     b->handles[free_slot] = h;
-    if (!general) b->sparse_tiles += tiles;
+    // (a member of another batch has kept the layout it had)
+    if (h->lane && h->lane_sparse) b->sparse_tiles += h->lgeo.n_slots / 32;
     if (!h->memberships) h->memberships = std::make_shared<int>(0);
     b->membership[free_slot] = h->memberships;
     ++*h->memberships;

@@ -125,3 +125,24 @@ def test_batches_step_many_sparse_tiles_with_the_general_kernels(tmp_path, cells
         s.handle.step(0.0, dt, 4)
     for s in solvers:
         assert np.abs(s.handle.get_state(0) - want).max() < 1e-12 * np.abs(want).max()
+
+
+def test_sparse_member_of_two_batches(tmp_path):
+    """The second batch takes the layout the first one steps the member with, and the room
+    among the tiles is what it was when it has left."""
+    path = write_mesh_file(tmp_path / "mesh.hpgem", [np.linspace(0.0, 1.0, 9)] * 2, True, 0.1)
+    solvers = [hpgem_b200.Advection(2, 3, [0.7, -0.4], tableau="RK4_4").readMeshFile(path) for _ in range(4)]
+    first, second = hpgem_b200.Batch(4), hpgem_b200.Batch(4)
+    kept = first.add(solvers[0], 1e-5, 0)
+    slots = [second.add(s, 1e-5, 0) for s in (solvers[1], solvers[2], solvers[0])]  # two of them fill the tiles
+    for _ in range(3):
+        second.remove(slots.pop())
+    assert second.num_classes == 0
+    second.add(solvers[1], 1e-5, 0)
+    second.add(solvers[2], 1e-5, 0)
+    second.add(solvers[3], 1e-5, 0)
+    members = {c["kind"]: c["members"] for c in second.class_info()}
+    assert members.pop("lane tables") == 2 and list(members.values()) == [1]
+    first.remove(kept)
+    first.close()
+    second.close()
